@@ -1,0 +1,491 @@
+// Prompt attention on tcgen05 tensor cores with the probabilities kept in TMEM: bf16 queries, keys and values, head sizes up to 256 in
+// multiples of 8 (queries / keys and values may differ), any group of query heads per key / value head up to 128, causal or not, a window of the
+// last keys; keys and values in 64-token cache pages, or as rows of the same ragged tokens (vision encoders, prompts without a cached prefix).
+//
+// One CTA = one KV head x up to two tiles of 128 (token, head of the group) rows of ONE sequence x one slice of its keys, in blocks of 128 keys.
+// Work items n = (block, tile) go through two TMEM score slots of 128 columns:
+//     S(n) = Q K^T        (tcgen05.mma kind::f16, M = 128, N = 128: with N = 64 the operand reads from shared memory would take longer than the
+//                          products; K = 16 steps up to the head size, so a head of 72 pays for 80)
+//     P(n) = exp2(S - m)  one warpgroup per tile; bf16 pairs written over S(n) in TMEM, the A operand of the second product
+//     O(t) += P(n) V      (N = head size up to the next multiple of 16; V read MN-major)
+// While one tile's softmax runs, the other tile's products do.  The products of a tile are issued by one thread in the order S, then PV(n) S(n+2) ..:
+// they complete in order, so S(n+2) may overwrite P(n) without a barrier.  Each tile has an issuer of its own: a barrier test costs the thread 300 cycles
+// once products are queued before it, and one issuer for both tiles was what bounded the kernel (4800 cycles for two 128 x 128 x 128 items, of which 2048
+// are products).  With a single tile (short sequences, value heads above 128 columns) the two slots are its consecutive key blocks.
+// kSplitP: probabilities stay 32-bit in effect: bf16 head and bf16 remainder (2^-17), two products against V.  Taken where the plain kernel this one
+// replaced kept them in fp32.
+// Shared memory: Q, then a ring of 16 KB slots (128 keys x 64 columns) shared by K and V, loaded in the order of first use; the chunks of a block's K
+// or V (a group) share one barrier.
+// Rows of V in front of the window or past the last visible key (pages that belong to nobody, rows of the next sequence) are zeroed in shared
+// memory before their product: 0 x inf there would reach the result.  Warp 0: TMA producer, 1 and 2: MMA issuers of tile 0 and 1, 3: that zeroing,
+// 4-7 / 8-11: softmax, rescale and epilogue of tile 0 / 1.  All waits are bounded.
+#include "ptx.cuh"
+#include "seq_tile.cuh"
+#include "tma_host.h"
+
+namespace ne {
+
+constexpr int kKernelFm = 27;
+constexpr int kFmBlk = 128;                    // keys per block
+constexpr int kFmSlot = kFmBlk * 128;          // 128 rows x 64 bf16 columns
+constexpr int kFmMaxSlots = 12;
+constexpr int kFmGroups = 16;                  // barriers of groups in flight; a group has at least one slot
+
+struct FmArgs {
+  const int* block_tables; int bt_stride;      // paged
+  const int* cu_seqlens_q; const int* context_lens; int num_seqs;      // context_lens null: the keys are the sequence's own tokens
+  int T, Hq, g, tq, tiles, splits;             // tq tokens per tile of g tq rows, up to `tiles` tiles per CTA
+  int nc, nv, ksteps, npv, dv;                 // 64-column chunks of K and V, K = 16 steps of the first product, N of the second, value columns
+  int rope_chunk;                              // chunks of K from this one on come from the rotary map, shared by the heads
+  int slots, window, causal, paged;
+  float scale_log2;
+  __nv_bfloat16* out;                          // [T, Hq, dv]
+  float* part; float* lse2;                    // [splits, T, Hq, dv], [splits, T, Hq] (splits > 1)
+};
+
+// (x, y) <- (x, y) scale + shift, and sum += (x, y): two fp32 operations in one instruction
+__device__ __forceinline__ void fma2(uint32_t& x, uint32_t& y, float scale, float shift) {
+  asm("{\n .reg .b64 a, b, c;\n mov.b64 a, {%0, %1};\n mov.b64 b, {%2, %2};\n mov.b64 c, {%3, %3};\n fma.rn.ftz.f32x2 a, a, b, c;\n mov.b64 {%0, %1}, a;\n}"
+      : "+r"(x), "+r"(y) : "f"(scale), "f"(shift));
+}
+__device__ __forceinline__ void add2(float (&sum)[2], uint32_t x, uint32_t y) {
+  asm("{\n .reg .b64 a, b;\n mov.b64 a, {%0, %1};\n mov.b64 b, {%2, %3};\n add.rn.ftz.f32x2 a, a, b;\n mov.b64 {%0, %1}, a;\n}" : "+f"(sum[0]), "+f"(sum[1]) : "r"(x), "r"(y));
+}
+__device__ __forceinline__ uint32_t ex2(uint32_t x) {
+  asm volatile("ex2.approx.ftz.f32 %0, %0;" : "+r"(x));      // volatile: in this order, back to back
+  return x;
+}
+
+// kWG: softmax warpgroups = most tiles per CTA
+template <int kWG, bool kSplitP>
+__global__ void __launch_bounds__(128 + 128 * kWG, 1)
+fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
+            const __grid_constant__ CUtensorMap r_map, const FmArgs a) {
+  pdl_wait();                     // dependent launch: nothing above this line touches global memory
+  extern __shared__ uint8_t smem_raw[];
+  // swizzled tiles need 1024-byte alignment; behind static shared memory the dynamic part starts on a 16-byte boundary
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sQ = smem;                                    // [tile][chunk][128 rows x 128 B]
+  uint8_t* sKV = sQ + kWG * a.nc * kFmSlot;
+  __shared__ uint64_t bars[2 * kFmGroups + 19];
+  __shared__ uint32_t s_tmem;
+  __shared__ int s_abort, s_seq, s_tok;
+  volatile int* abort_flag = &s_abort;
+  const uint32_t b_full = smem_u32(bars), b_empty = b_full + 8 * kFmGroups, b_q = b_empty + 8 * kFmGroups, b_s = b_q + 8, b_p = b_s + 16, b_pv = b_p + 16,
+                 b_go = b_pv + 16, b_fix = b_go + 16, b_turn = b_fix + 16;
+  const int warp = threadIdx.x >> 5;
+  const int hkv = blockIdx.y, split = blockIdx.z;
+  if (warp == 0) {
+    int seq, tok;
+    // later tiles of a sequence see more keys: they start first
+    find_seq_tile(a.cu_seqlens_q, a.num_seqs, a.tq * a.tiles, (int)(gridDim.x - 1 - blockIdx.x), seq, tok);
+    if (lane_id() == 0) { s_seq = seq; s_tok = tok; }
+  }
+  if (warp == 2) { tmem_alloc(smem_u32(&s_tmem), 512); tmem_relinquish(); }
+  __syncthreads();
+  const int seq = s_seq, tok0 = s_tok;
+
+  // geometry (uniform over the CTA)
+  int nt = 1, nblk = 0, blk0 = 0, n_tok = 0, base_limit = -1, vis_lo = 0, vis_hi = -1, k_beg = 0;
+  if (seq >= 0) {
+    const int q_beg = a.cu_seqlens_q[seq], q_len = a.cu_seqlens_q[seq + 1] - q_beg, ctx = a.context_lens ? a.context_lens[seq] : q_len;
+    n_tok = min(a.tq * a.tiles, q_beg + q_len - tok0);
+    nt = n_tok > a.tq ? 2 : 1;
+    k_beg = q_beg;
+    base_limit = a.causal ? ctx - q_len + (tok0 - q_beg) : ctx - 1;          // last key visible to the tile's first token
+    vis_hi = a.causal ? base_limit + n_tok - 1 : base_limit;                  // ... to any of its tokens
+    vis_lo = a.window > 0 ? max(0, base_limit - a.window + 1) : 0;
+    const int first = vis_lo / kFmBlk, total = vis_hi >= 0 ? vis_hi / kFmBlk + 1 - first : 0;
+    const int per_split = (total + a.splits - 1) / a.splits;
+    blk0 = first + split * per_split;
+    nblk = max(0, min(total, (split + 1) * per_split) - split * per_split);
+  }
+  const int items = nblk * nt;
+  if (threadIdx.x == 32) {
+    for (int i = 0; i < kFmGroups; i++) { mbar_init(b_full + 8 * i, 1); mbar_init(b_empty + 8 * i, nt); }
+    mbar_init(b_q, 1);
+    for (int i = 0; i < 2; i++) {
+      mbar_init(b_s + 8 * i, 1); mbar_init(b_p + 8 * i, 4); mbar_init(b_pv + 8 * i, 1); mbar_init(b_go + 8 * i, 1); mbar_init(b_fix + 8 * i, 32);
+    }
+    for (int i = 0; i < 8; i++) mbar_init(b_turn + 8 * i, 1);
+    s_abort = 0;
+    mbar_fence_init();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_trigger();                  // behind the TMEM allocation: a CTA of the next grid never holds columns this grid waits for
+  const uint32_t tmem = s_tmem;   // S/P slots at columns 0 and 128, O of tile t at 256 + 128 t
+  const bool fix_lo = nblk > 0 && blk0 * kFmBlk < vis_lo, fix_hi = nblk > 0 && (blk0 + nblk) * kFmBlk - 1 > vis_hi;
+
+  if (warp == 0) {
+    if (items > 0 && elect_one()) {
+      mbar_expect_tx(b_q, nt * a.nc * a.g * a.tq * 128);
+      for (int t = 0; t < nt; t++)
+        for (int c = 0; c < a.nc; c++) tma_load_3d(smem_u32(sQ + (t * a.nc + c) * kFmSlot), &q_map, b_q, c * 64, hkv * a.g, tok0 + t * a.tq);
+      int s = 0, group = 0, tail = 0, room = a.slots;      // groups are released in the order of loading
+      auto size_of = [&](int g) { return (nt == 2 ? (g & 1) : g == 2 * nblk - 1 || (g > 0 && !(g & 1))) ? a.nv : a.nc; };
+      const int* bt = a.block_tables + (long long)seq * a.bt_stride;
+      auto load = [&](int j, bool v) -> bool {
+        const int key0 = (blk0 + j) * kFmBlk;
+        int pg[2] = {0, 0};
+        if (a.paged)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {      // pages without a visible key (their table entry may be anything) read one that has
+            pg[h] = bt[min(max(key0 / 64 + h, vis_lo / 64), vis_hi / 64)];
+            if (!NE_INDEX_OK(pg[h], BK_CACHE_PAGES, kKernelFm, __LINE__)) pg[h] = 0;
+          }
+        const int n = v ? a.nv : a.nc;
+        for (; room < n; tail++) {
+          if (!mbar_wait(b_empty + 8 * (tail % kFmGroups), (tail / kFmGroups) & 1, abort_flag, kKernelFm, 100)) return false;
+          room += size_of(tail);
+        }
+        room -= n;
+        const uint32_t bar = b_full + 8 * (group++ % kFmGroups);
+        mbar_expect_tx(bar, n * kFmSlot);
+        for (int c = 0; c < n; c++) {
+          const uint32_t dst = smem_u32(sKV + s * kFmSlot);
+          if (a.paged) {
+            tma_load_4d(dst, v ? &v_map : &k_map, bar, c * 64, hkv, 0, pg[0]);
+            tma_load_4d(dst + kFmSlot / 2, v ? &v_map : &k_map, bar, c * 64, hkv, 0, pg[1]);
+          } else if (!v && c >= a.rope_chunk) {
+            tma_load_2d(dst, &r_map, bar, (c - a.rope_chunk) * 64, k_beg + key0);
+          } else {
+            tma_load_3d(dst, v ? &v_map : &k_map, bar, c * 64, hkv, k_beg + key0);      // rows past the tensor's end are zero-filled
+          }
+          if (++s == a.slots) s = 0;
+        }
+        if (v && j == 0 && fix_lo) mbar_arrive(b_go);
+        if (v && j == nblk - 1 && fix_hi) mbar_arrive(b_go + 8);
+        return true;
+      };
+      bool ok = load(0, false);
+      if (ok && nt == 1 && nblk > 1) ok = load(1, false);
+      for (int j = 0; ok && j < nblk; j++) {
+        const int next = j + (nt == 2 ? 1 : 2);
+        ok = load(j, true) && (next >= nblk || load(next, false));
+      }
+    }
+  } else if (warp <= 2) {
+    const int t = warp - 1;       // the issuer's tile
+    if (t < nt && items > 0 && elect_one()) {
+      constexpr uint32_t kIdS = make_idesc(FMT_BF16, FMT_BF16, 128, kFmBlk);
+      const uint32_t id_pv = make_idesc(FMT_BF16, FMT_BF16, 128, (uint32_t)a.npv, 0, 1);      // B (= V) is MN-major
+      // descriptors of the operands' first tiles; others by adding their distance (in units of 16 bytes)
+      constexpr uint32_t kTile = kFmSlot >> 4;
+      const uint64_t dq = make_smem_desc(smem_u32(sQ), 16, 1024, SW_128B) + t * a.nc * kTile, dk = make_smem_desc(smem_u32(sKV), 16, 1024, SW_128B),
+                     dv = make_smem_desc(smem_u32(sKV), kFmSlot, 1024, SW_128B);
+      const uint32_t o = tmem + 256 + t * 128;
+      // first slots of the groups in the order of loading (no division: its reciprocal would wait behind the softmax's exponentials)
+      int s = 0, group = 0;
+      auto take = [&](int n, int where, int& first, int& bar) -> bool {
+        if (!mbar_wait(b_full + 8 * (group % kFmGroups), (group / kFmGroups) & 1, abort_flag, kKernelFm, where)) return false;
+        first = s; bar = group++ % kFmGroups;
+        s += n;
+        if (s >= a.slots) s -= a.slots;
+        return true;
+      };
+      int k0 = 0, kb = 0, v0 = 0, vb = 0;
+      auto scores = [&](int n) {
+        tc_fence_after();
+        const uint32_t d = tmem + (n & 1) * kFmBlk;
+        int ks = k0;
+        for (int c = 0; c < a.nc; c++) {
+          const uint64_t qa = dq + c * kTile, ka = dk + ks * kTile;
+          const int steps = a.ksteps - 4 * c;
+          umma_f16(d, qa, ka, kIdS, c != 0);
+          if (steps > 1) umma_f16(d, qa + 2, ka + 2, kIdS, 1);
+          if (steps > 2) umma_f16(d, qa + 4, ka + 4, kIdS, 1);
+          if (steps > 3) umma_f16(d, qa + 6, ka + 6, kIdS, 1);
+          if (++ks == a.slots) ks = 0;
+        }
+        tc_commit(b_s + 8 * (n & 1));
+        tc_commit(b_empty + 8 * kb);
+      };
+      bool ok = mbar_wait(b_q, 0, abort_flag, kKernelFm, 200) && take(a.nc, 210, k0, kb);
+      if (ok) scores(t);
+      if (ok && nt == 1 && nblk > 1) {
+        ok = take(a.nc, 211, k0, kb);
+        if (ok) scores(1);
+      }
+      for (int j = 0; ok && j < nblk; j++) {
+        const int n = j * nt + t, next = nt == 2 ? j + 1 : j + 2;      // item n + 2 is block `next` of this tile
+        // the next products' operands are waited for while the softmax works
+        ok = take(a.nv, 220, v0, vb) && (next >= nblk || take(a.nc, 212, k0, kb));
+        if (ok && j == 0 && fix_lo) ok = mbar_wait(b_fix, 0, abort_flag, kKernelFm, 221);
+        if (ok && j == nblk - 1 && fix_hi) ok = mbar_wait(b_fix + 8, 0, abort_flag, kKernelFm, 222);
+        if (!ok || !mbar_wait(b_p + 8 * (n & 1), (n >> 1) & 1, abort_flag, kKernelFm, 230)) break;
+        tc_fence_after();
+        const uint32_t p = tmem + (n & 1) * kFmBlk;
+        // the chunks of V lie in consecutive ring slots; where they wrap around the ring's end, the product is issued in two column ranges
+        const int head = min(a.nv, a.slots - v0);
+        const uint64_t va = dv + v0 * kTile;
+        if (head == a.nv) {
+#pragma unroll
+          for (int x = 0; x < (kSplitP ? 2 : 1); x++)
+#pragma unroll
+            for (int ks = 0; ks < 8; ks++) umma_f16_ts(o, p + x * 64 + ks * 8, va + ks * 128, id_pv, (x | ks) ? 1u : (uint32_t)(j != 0));
+        } else {
+          const uint32_t id_a = make_idesc(FMT_BF16, FMT_BF16, 128, (uint32_t)head * 64, 0, 1), id_b = make_idesc(FMT_BF16, FMT_BF16, 128, (uint32_t)(a.npv - head * 64), 0, 1);
+#pragma unroll
+          for (int x = 0; x < (kSplitP ? 2 : 1); x++)
+#pragma unroll
+            for (int ks = 0; ks < 8; ks++) {
+              umma_f16_ts(o, p + x * 64 + ks * 8, va + ks * 128, id_a, (x | ks) ? 1u : (uint32_t)(j != 0));
+              umma_f16_ts(o + head * 64, p + x * 64 + ks * 8, dv + ks * 128, id_b, (x | ks) ? 1u : (uint32_t)(j != 0));
+            }
+        }
+        tc_commit(b_pv + 8 * (n & 1));
+        tc_commit(b_empty + 8 * vb);
+        if (next < nblk) scores(n + 2);
+      }
+    }
+  } else if (warp < 4) {
+    for (int w = 0; w < 2; w++) {
+      if (!(w ? fix_hi : fix_lo)) continue;
+      const int j = w ? nblk - 1 : 0, key0 = (blk0 + j) * kFmBlk;
+      // group and first slot of the block's V in the order of loading
+      const int g = nt == 2 ? 2 * j + 1 : min(j + 2, nblk) + j, p0 = nt == 2 ? j * (a.nc + a.nv) + a.nc : min(j + 2, nblk) * a.nc + j * a.nv;
+      // once its loads are under way the phase waited for is the current one
+      if (mbar_wait(b_go + 8 * w, 0, abort_flag, kKernelFm, 400) && mbar_wait(b_full + 8 * (g % kFmGroups), (g / kFmGroups) & 1, abort_flag, kKernelFm, 410))
+        for (int i = (int)lane_id(); i < a.nv * kFmBlk; i += 32) {
+          const int key = key0 + (i & (kFmBlk - 1));
+          if (w ? key > vis_hi : key < vis_lo) {
+            uint4* dst = reinterpret_cast<uint4*>(sKV + ((p0 + (i >> 7)) % a.slots) * kFmSlot + (i & (kFmBlk - 1)) * 128);
+#pragma unroll
+            for (int x = 0; x < 8; x++) dst[x] = make_uint4(0, 0, 0, 0);
+          }
+        }
+      fence_proxy_async_smem();
+      mbar_arrive(b_fix + 8 * w);
+    }
+  } else {
+    const int t = (warp - 4) >> 2, wq = warp & 3, row = wq * 32 + (int)lane_id();
+    const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
+    const int tl = t * a.tq + row / a.g, head = hkv * a.g + row % a.g;        // token of the CTA's tiles
+    const bool row_ok = row < a.g * a.tq && tl < n_tok;
+    const int limit = row_ok ? (a.causal ? base_limit + tl : base_limit) : -1;
+    const int lowest = a.window > 0 ? limit - a.window + 1 : 0;
+    const uint32_t tmem_o = tmem + 256 + t * 128 + lane_addr;
+    float m_run = -INFINITY, l_run = 0.f;
+    bool ok = true;
+    int last = -1;
+    for (int n = t; ok && t < nt && n < items; n += nt) {
+      const int key0 = (blk0 + (nt == 2 ? n >> 1 : n)) * kFmBlk;
+      const uint32_t ts = tmem + (n & 1) * kFmBlk + lane_addr;
+      if (!mbar_wait(b_s + 8 * (n & 1), (n >> 1) & 1, abort_flag, kKernelFm, 300)) { ok = false; break; }
+      tc_fence_after();
+      __syncwarp();
+      uint32_t r[128];
+#pragma unroll
+      for (int c = 0; c < 4; c++) tmem_ld_32x32b_x32(ts + c * 32, *reinterpret_cast<uint32_t(*)[32]>(r + c * 32));
+      tc_wait_ld();
+      if (key0 + kFmBlk - 1 > limit || key0 < lowest) {
+#pragma unroll
+        for (int j = 0; j < 128; j++)
+          if (key0 + j > limit || key0 + j < lowest) r[j] = 0xff800000u;
+      }
+#ifdef NE_DEBUG_BOUNDS
+      if (a.paged)                             // the keys of a page that is none take no part
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int pg = key0 / 64 + h;
+          if (pg <= vis_hi / 64 && !NE_INDEX_OK(a.block_tables[(long long)seq * a.bt_stride + max(pg, vis_lo / 64)], BK_CACHE_PAGES, kKernelFm, __LINE__)) {
+#pragma unroll
+            for (int j = 0; j < 64; j++) r[h * 64 + j] = 0xff800000u;
+          }
+        }
+#endif
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int j = 0; j < 128; j++) mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(r[j]));
+      // the reference is a whole power of two: rescaling by it is exact, and a probability rounds alike whatever the blocks are
+      const float m_tile = ceilf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * a.scale_log2);
+      // lazy rescaling: the reference maximum only moves when the block's maximum exceeds it by more than 2^8
+      const bool first_valid = m_run == -INFINITY;
+      const float m_new = (first_valid || m_tile > m_run + 8.f) ? fmaxf(m_run, m_tile) : m_run;
+      const float alpha = (m_new == -INFINITY || first_valid) ? 1.f : exp2f(m_run - m_new);
+      const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
+      float ps[2] = {0.f, 0.f};
+      __syncwarp();                          // rows at a limit took a branch of their own
+      // the two tiles take turns at the exponentials (warps of one scheduler in pairs): left alone they fall into step, and then neither tile's
+      // products run beside the other's softmax
+      const int turn = n >> 1;
+      if (nt == 2 && (t || turn) && !mbar_wait(b_turn + 8 * (t * 4 + wq), (t ? turn : turn - 1) & 1, abort_flag, kKernelFm, 330)) { ok = false; break; }
+      // 32 columns at a time; the next ones' exponentials are under way while these are packed and stored
+      auto exps = [&](int c) {
+#pragma unroll
+        for (int j = 0; j < 16; j++) fma2(r[c * 32 + 2 * j], r[c * 32 + 2 * j + 1], a.scale_log2, neg_m);
+#pragma unroll
+        for (int j = 0; j < 32; j++) r[c * 32 + j] = ex2(r[c * 32 + j]);
+      };
+      exps(0);
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        if (c < 3) exps(c + 1);
+        uint32_t* x = r + c * 32;
+        uint32_t hi[16];
+        if constexpr (kSplitP) {
+          uint32_t lo[16];
+#pragma unroll
+          for (int j = 0; j < 16; j++) {       // the head is cut off, not rounded: the remainder takes the difference either way
+            hi[j] = __byte_perm(x[2 * j], x[2 * j + 1], 0x7632);
+            add2(ps, x[2 * j], x[2 * j + 1]);
+            lo[j] = pack_bf16x2(__uint_as_float(x[2 * j]) - __uint_as_float(x[2 * j] & 0xffff0000u), __uint_as_float(x[2 * j + 1]) - __uint_as_float(x[2 * j + 1] & 0xffff0000u));
+          }
+          tmem_st_32x32b_x16(ts + 64 + c * 16, lo);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; j++) {       // sum what the product will see, so numerator and denominator stay consistent
+            hi[j] = pack_bf16x2(__uint_as_float(x[2 * j]), __uint_as_float(x[2 * j + 1]));
+            add2(ps, hi[j] << 16, hi[j] & 0xffff0000u);
+          }
+        }
+        tmem_st_32x32b_x16(ts + c * 16, hi);
+      }
+      __syncwarp();
+      if (nt == 2 && lane_id() == 0) mbar_arrive(b_turn + 8 * ((t ^ 1) * 4 + wq));
+      l_run = l_run * alpha + (ps[0] + ps[1]);
+      m_run = m_new;
+      if (last >= 0 && __any_sync(0xffffffffu, alpha < 1.f)) {
+        if (!mbar_wait(b_pv + 8 * (last & 1), (last >> 1) & 1, abort_flag, kKernelFm, 310)) { ok = false; break; }
+        tc_fence_after();
+#pragma unroll 1
+        for (int cblk = 0; cblk < (a.npv + 15) / 16; cblk++) {
+          uint32_t o[16];
+          tmem_ld_32x32b_x16(tmem_o + cblk * 16, o);
+          tc_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 16; j++) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
+          tmem_st_32x32b_x16(tmem_o + cblk * 16, o);
+        }
+      }
+      tc_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane_id() == 0) mbar_arrive(b_p + 8 * (n & 1));
+      last = n;
+    }
+    if (ok && last >= 0) ok = mbar_wait(b_pv + 8 * (last & 1), (last >> 1) & 1, abort_flag, kKernelFm, 320);
+    const bool have = ok && last >= 0;
+    const long long rows = (long long)a.T * a.Hq, orow = row_ok ? (long long)(tok0 + tl) * a.Hq + head : 0;
+    if (have) tc_fence_after();
+    __syncwarp();
+    const float inv = have && l_run > 0.f ? 1.f / l_run : 0.f;
+#pragma unroll 1
+    for (int cblk = 0; cblk < (a.npv + 15) / 16; cblk++) {
+      uint32_t o[16];
+      __syncwarp();                          // the lanes of rows outside the tile skip the stores below
+      if (have) {
+        tmem_ld_32x32b_x16(tmem_o + cblk * 16, o);
+        tc_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; j++) o[j] = __float_as_uint(__uint_as_float(o[j]) * inv);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; j++) o[j] = 0u;
+      }
+      if (!row_ok) continue;
+#pragma unroll
+      for (int v = 0; v < 2; v++) {          // dv is a multiple of 8
+        const int col = cblk * 16 + v * 8;
+        if (col >= a.dv) continue;
+        const float* f = reinterpret_cast<const float*>(o + v * 8);
+        if (a.splits == 1) {
+          *reinterpret_cast<uint4*>(a.out + orow * a.dv + col) = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+        } else {
+          float* dst = a.part + ((long long)split * rows + orow) * a.dv + col;
+          *reinterpret_cast<float4*>(dst) = make_float4(f[0], f[1], f[2], f[3]);
+          *reinterpret_cast<float4*>(dst + 4) = make_float4(f[4], f[5], f[6], f[7]);
+        }
+      }
+    }
+    if (a.splits > 1 && row_ok) a.lse2[(long long)split * rows + orow] = (have && l_run > 0.f) ? m_run + log2f(l_run) : -INFINITY;
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag && threadIdx.x == 0) for (int i = 0; i < 2000; i++) __nanosleep(1000);      // copies in flight
+  __syncthreads();
+  if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, 512); }
+}
+
+constexpr int kFmSmem = 232448 - 1024;         // dynamic shared memory limit of a block less the static part
+
+template <int kWG, bool kSplitP>
+static int fmha_launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const CUtensorMap& r, const FmArgs& a, int grid_x, int heads, cudaStream_t st) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(fmha_kernel<kWG, kSplitP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFmSmem);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  return (int)launch_pdl(fmha_kernel<kWG, kSplitP>, dim3((unsigned)grid_x, (unsigned)heads, (unsigned)a.splits), dim3(128 + 128 * kWG),
+                         (size_t)(kWG * a.nc + a.slots) * kFmSlot + 1024, st, q, k, v, r, a);
+}
+
+}  // namespace ne
+
+using namespace ne;
+
+// Query tokens per CTA tile set (0: sizes this kernel does not cover).  rows: new tokens of the longest sequence, where known (0: unknown).
+extern "C" int ne_fmha_plan(int g, int D, int Dv, int rows, int* tiles) {
+  if (g < 1 || g > 128 || D < 8 || D > 256 || D % 8 || Dv < 8 || Dv > 256 || Dv % 8) return 0;
+  const int tq = 128 / g;
+  // two tiles: one's softmax runs beside the other's products; TMEM holds two accumulators of up to 128 columns, shared memory two Q tiles of up to 192
+  *tiles = Dv <= 128 && D <= 192 && (rows == 0 || rows > tq) ? 2 : 1;
+  return tq * *tiles;
+}
+
+// q [T, Hq, D] with row stride q_ld (elements; heads D apart), keys / values either pages k, v [num_blocks, 64, Hkv, D or Dv] contiguous (block_tables
+// not null) or rows [T, Hkv, D or Dv] with row strides k_ld, v_ld; k_rope not null (ragged only): the last D - Dk_nope columns of every head's key are the
+// row k_rope [T, D - Dk_nope] (row stride r_ld), k_nope heads k_head apart.  context_lens null: keys are the sequence's own tokens.
+// split_p: probabilities as two bf16 terms.  splits > 1: part / lse2 as ne_attn_merge takes them.
+extern "C" int ne_fmha(const void* q, long long q_ld, const void* k, long long k_ld, int k_dim, const void* k_rope, long long r_ld, const void* v, long long v_ld,
+                       int num_blocks, const int* block_tables, int bt_stride, const int* cu_seqlens_q, const int* context_lens, int num_seqs, int T, int Hq,
+                       int Hkv, int D, int Dv, int tiles, int grid_x, int splits, int window, int causal, float scale, int split_p, void* out, float* part,
+                       float* lse2, cudaStream_t st) {
+  if (T <= 0) return 0;
+  if (Hkv < 1 || Hq % Hkv || splits < 1 || (splits > 1 && (!part || !lse2)) || grid_x < 1 || Hkv > 65535) return 1001;
+  int most = 0;
+  if (!ne_fmha_plan(Hq / Hkv, D, Dv, 0, &most) || tiles < 1 || tiles > most) return 1002;
+  if (q_ld % 8 || q_ld < (long long)Hq * D || (block_tables == nullptr && (k_ld % 8 || v_ld % 8)) || (k_rope && (block_tables || r_ld % 8 || k_dim % 64 || k_dim >= D))) return 1003;
+  FmArgs a;
+  a.g = Hq / Hkv; a.tq = 128 / a.g; a.tiles = tiles; a.splits = splits; a.T = T; a.Hq = Hq;
+  a.nc = (D + 63) / 64; a.nv = (Dv + 63) / 64; a.ksteps = (D + 15) / 16; a.npv = (Dv + 15) / 16 * 16; a.dv = Dv;
+  a.rope_chunk = k_rope ? k_dim / 64 : a.nc;
+  a.slots = (kFmSmem - 1024) / kFmSlot - tiles * a.nc;
+  if (a.slots > kFmMaxSlots) a.slots = kFmMaxSlots;
+  if (a.slots < a.nc + a.nv) return 1004;                           // a block's K waits for its V, and the next block's K beside it
+  a.window = window > 0 ? window : 0; a.causal = causal; a.paged = block_tables != nullptr;
+  a.block_tables = block_tables; a.bt_stride = bt_stride; a.cu_seqlens_q = cu_seqlens_q; a.context_lens = context_lens; a.num_seqs = num_seqs;
+  a.scale_log2 = scale * 1.4426950408889634f; a.out = (__nv_bfloat16*)out; a.part = part; a.lse2 = lse2;
+  CUtensorMap mq, mk, mv, mr;
+  {
+    uint64_t dims[3] = {(uint64_t)D, (uint64_t)Hq, (uint64_t)T}, strides[2] = {(uint64_t)D * 2, (uint64_t)q_ld * 2};
+    uint32_t box[3] = {64, (uint32_t)a.g, (uint32_t)a.tq};
+    int rc = make_tmap(&mq, q, TMA_BF16, 3, dims, strides, box, TMA_SW_128); if (rc) return 2000 + rc;
+  }
+  for (int w = 0; w < 2; w++) {
+    const uint64_t d = w ? Dv : (k_rope ? k_dim : D);
+    int rc;
+    if (a.paged) {
+      uint64_t dims[4] = {d, (uint64_t)Hkv, 64, (uint64_t)num_blocks}, strides[3] = {d * 2, (uint64_t)Hkv * d * 2, 64 * (uint64_t)Hkv * d * 2};
+      uint32_t box[4] = {64, 1, 64, 1};
+      rc = make_tmap(w ? &mv : &mk, w ? v : k, TMA_BF16, 4, dims, strides, box, TMA_SW_128);
+    } else {
+      uint64_t dims[3] = {d, (uint64_t)Hkv, (uint64_t)T}, strides[2] = {d * 2, (uint64_t)(w ? v_ld : k_ld) * 2};
+      uint32_t box[3] = {64, 1, kFmBlk};
+      rc = make_tmap(w ? &mv : &mk, w ? v : k, TMA_BF16, 3, dims, strides, box, TMA_SW_128);
+    }
+    if (rc) return 2100 + rc;
+  }
+  mr = mk;
+  if (k_rope) {
+    uint64_t dims[2] = {(uint64_t)(D - k_dim), (uint64_t)T}, strides[1] = {(uint64_t)r_ld * 2};
+    uint32_t box[2] = {64, kFmBlk};
+    int rc = make_tmap(&mr, k_rope, TMA_BF16, 2, dims, strides, box, TMA_SW_128); if (rc) return 2200 + rc;
+  }
+  if (tiles == 2) return split_p ? fmha_launch<2, true>(mq, mk, mv, mr, a, grid_x, Hkv, st) : fmha_launch<2, false>(mq, mk, mv, mr, a, grid_x, Hkv, st);
+  return split_p ? fmha_launch<1, true>(mq, mk, mv, mr, a, grid_x, Hkv, st) : fmha_launch<1, false>(mq, mk, mv, mr, a, grid_x, Hkv, st);
+}

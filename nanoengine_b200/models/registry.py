@@ -70,7 +70,7 @@ def _gipozen():
 
 
 # kernel sources (stems under csrc/) of the architectures that can be served from a partial build; None = all of them
-_KERNELS = {"Tuvutar": ("gemm", "gemm_simt", "residual", "elementwise", "attn_generic", "gqa_bf16", "mla_bf16", "delta"),
+_KERNELS = {"Tuvutar": ("gemm", "gemm_simt", "residual", "elementwise", "attn_generic", "gqa_bf16", "fmha", "mla_bf16", "delta"),
             "Filasun": ("gemm", "gemm_simt", "residual", "elementwise", "attn_generic", "gqa_biased", "linattn", "linattn_tc"),
             "Sapanex": ("gemm", "gemm_simt", "residual", "elementwise", "attn_generic", "gqa_biased", "pooled", "general_delta"),
             "Gipozen": ("gemm", "gemm_simt", "residual", "elementwise", "attn_generic", "gqa_biased", "shortconv", "moe")}

@@ -162,9 +162,50 @@ def mla_attention_paged(q, cache, block_tables, cu_seqlens_q, context_lens, scal
     return out
 
 
+PROMPT_TC_CALLS = [0]        # launches of the tensor-core prompt attention kernel
+
+
+def _fmha(q, k, v, cu, scale, causal, split_p, block_tables=None, context_lens=None, window=0, k_rope=None, one_token=False):
+    """The tcgen05 prompt kernel; shapes checked by the caller.  Returns None for sizes it does not cover."""
+    T, Hq, D = q.shape
+    paged = block_tables is not None
+    Hkv, Dv = (k.shape[2], v.shape[3]) if paged else (k.shape[1], v.shape[2])
+    B = cu.numel() - 1
+    lib = _k.lib()
+    tiles = _c.c_int(0)
+    rows = lib.ne_fmha_plan(_c.c_int(Hq // Hkv), _c.c_int(D), _c.c_int(Dv), _c.c_int(1 if one_token else 0), _c.byref(tiles))
+    if not rows:
+        return None
+    grid = min(T, T // rows + B)
+    S = 1
+    if paged and grid * Hkv < _sms() // 2:             # few CTAs (small decode batches, short prompts): slice the keys, blocks of 128
+        pages = block_tables.shape[1] if window <= 0 else min(block_tables.shape[1], (window + rows + 126) // 64 + 1)
+        S = max(1, min(_sms() // (grid * Hkv), max(1, pages // 4), 16))
+    out = torch.empty(T, Hq, Dv, dtype=torch.bfloat16, device=q.device)
+    part = lse2 = None
+    if S > 1:
+        part = torch.empty(S, T, Hq, Dv, dtype=torch.float32, device=q.device)
+        lse2 = torch.empty(S, T, Hq, dtype=torch.float32, device=q.device)
+    _k._ck(lib.ne_fmha(_k._p(q), _c.c_longlong(q.stride(0)), _k._p(k), _c.c_longlong(k.stride(0)), _c.c_int(k.shape[-1]), _k._p(k_rope),
+                       _c.c_longlong(0 if k_rope is None else k_rope.stride(0)), _k._p(v), _c.c_longlong(v.stride(0)), _c.c_int(k.shape[0]), _k._p(block_tables),
+                       _c.c_int(block_tables.stride(0) if paged else 0), _k._p(cu), _k._p(context_lens), _c.c_int(B), _c.c_int(T), _c.c_int(Hq), _c.c_int(Hkv),
+                       _c.c_int(D), _c.c_int(Dv), tiles, _c.c_int(grid), _c.c_int(S), _c.c_int(max(0, int(window))), _c.c_int(1 if causal else 0), _c.c_float(scale),
+                       _c.c_int(1 if split_p else 0), _k._p(out), _k._p(part), _k._p(lse2), _k._st()), "ne_fmha")
+    PROMPT_TC_CALLS[0] += 1
+    if S > 1:
+        _k._ck(lib.ne_attn_merge(_k._p(part), _k._p(lse2), _k._p(out), _c.c_int(S), _c.c_longlong(T * Hq), _c.c_int(Dv), _c.c_int(Dv), _k._st()),
+               "ne_attn_merge")
+    return out
+
+
+def _rows16(t):
+    """Rows of [T, H, D] that TMA can address: heads D apart, 16-byte aligned."""
+    return t.stride(2) == 1 and t.stride(1) == t.shape[2] and t.stride(0) % 8 == 0 and t.stride(0) >= t.shape[1] * t.shape[2] and t.data_ptr() % 16 == 0
+
+
 def gqa_attention_paged(q, k_cache, v_cache, block_tables, cu_seqlens_q, context_lens, scale, window: int = 0):
-    """`window` > 0: every query sees only its last `window` key positions (sliding-window layers); those layers and head
-    dims other than 128 run on the generic kernel."""
+    """`window` > 0: every query sees only its last `window` key positions (sliding-window layers).  bf16 caches of 64-token pages: tensor cores.  Those
+    layers, and head sizes other than 128, keep their probabilities in 32-bit (two bf16 terms); other caches run on the generic kernel."""
     T, Hq, D = q.shape
     Hkv = k_cache.shape[2]
     lib = _k.lib()
@@ -174,12 +215,17 @@ def gqa_attention_paged(q, k_cache, v_cache, block_tables, cu_seqlens_q, context
     if T == 0:
         return out
     group = Hq // Hkv
-    if (D == 128 and window <= 0 and k_cache.dtype == torch.bfloat16 and v_cache.dtype == torch.bfloat16 and k_cache.shape[1] == 64 and Hq % Hkv == 0
-            and group <= 128 and group & (group - 1) == 0 and k_cache.is_contiguous() and v_cache.is_contiguous()):
-        # tcgen05 kernel: one CTA per (kv head, tile of 128 (token, head) rows, key slice)
+    B = cl.numel()
+    pages64 = (k_cache.dtype == torch.bfloat16 and v_cache.dtype == torch.bfloat16 and k_cache.shape[1] == 64 and Hq % Hkv == 0 and group <= 128
+               and k_cache.is_contiguous() and v_cache.is_contiguous())
+    if D == 128 and window <= 0 and pages64 and group & (group - 1) == 0:
         q = q.contiguous()
+        if T > B:                                      # some sequence has more than one new token
+            got = _fmha(q, k_cache, v_cache, cu, scale, True, False, bt, cl)
+            if got is not None:
+                return got
+        # tcgen05 kernel: one CTA per (kv head, tile of 128 (token, head) rows, key slice)
         tq = 128 // group
-        B = cl.numel()
         max_tiles = min(T, T // tq + B)
         S = 1
         if max_tiles * Hkv < 74:                       # few CTAs (small decode batches): slice the keys
@@ -196,6 +242,10 @@ def gqa_attention_paged(q, k_cache, v_cache, block_tables, cu_seqlens_q, context
                    "ne_attn_merge")
         return out
     assert group % 4 == 0 or group == 1 and Hq % 4 == 0 or Hkv == Hq, "query heads per kv head must be a multiple of 4"
+    if pages64 and scale > 0 and k_cache.shape[3] == v_cache.shape[3] == D and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0 and D % 8 == 0:
+        got = _fmha(q if _rows16(q) else q.clone(memory_format=torch.contiguous_format), k_cache, v_cache, cu, scale, True, True, bt, cl, window, one_token=T <= B)
+        if got is not None:
+            return got
     _k._ck(lib.ne_attn_generic(_k._p(q), _c.c_longlong(q.stride(0)), _c.c_int(q.stride(1)), _k._p(k_cache), _k._p(v_cache),
                                _c.c_longlong(Hkv * D), _c.c_int(D), _c.c_int(group), _k._p(bt), _c.c_int(bt.stride(0)), _c.c_int(k_cache.shape[1]),
                                _k._p(cu), _k._p(cl), _c.c_int(cl.numel()), _k._p(None), _c.c_int(0), _k._p(out), _c.c_longlong(Hq * D), _c.c_int(D),
@@ -316,15 +366,21 @@ def differential_attention(q, k_cache, v_cache, block_tables, cu_seqlens_q, cont
 
 def attention_varlen(q, k, v, cu_seqlens, scale, causal: bool = False):
     """Attention over ragged sequences without a paged cache: q, k, v [T, H, D] of the same tokens, sequence i owns rows
-    [cu[i], cu[i+1]).  Runs on the generic kernel, which addresses k / v as a one-row-per-page cache through a table of row
-    numbers (no copy); any head dim up to 640.  Used by the vision encoder (non-causal)."""
+    [cu[i], cu[i+1]).  Head sizes up to 256 in multiples of 8: tensor cores, probabilities in 32-bit (two bf16 terms).  Others run on the generic
+    kernel, which addresses k / v as a one-row-per-page cache through a table of row numbers (no copy); any head dim up to 640.
+    Used by the vision encoder (non-causal)."""
     T, H, D = q.shape
     q = q if (q.dtype == torch.bfloat16 and q.stride(-1) == 1) else q.to(torch.bfloat16).contiguous()
-    k, v = k.to(torch.bfloat16).contiguous(), v.to(torch.bfloat16).contiguous()
-    out = torch.empty(T, H, D, dtype=torch.bfloat16, device=q.device)
+    k, v = k.to(torch.bfloat16), v.to(torch.bfloat16)
     if T == 0:
-        return out
+        return torch.empty(T, H, D, dtype=torch.bfloat16, device=q.device)
     cu = _i32(cu_seqlens)
+    if scale > 0 and D % 8 == 0 and D <= 256 and k.shape == q.shape and v.shape == q.shape:
+        got = _fmha(*[t if _rows16(t) else t.clone(memory_format=torch.contiguous_format) for t in (q, k, v)], cu, scale, causal, True)
+        if got is not None:
+            return got
+    k, v = k.contiguous(), v.contiguous()
+    out = torch.empty(T, H, D, dtype=torch.bfloat16, device=q.device)
     lens = (cu[1:] - cu[:-1])
     B = lens.numel()
     max_len = int(lens.max())

@@ -1,0 +1,91 @@
+"""The tensor-core prompt attention kernel through its entry points: edges of the 128-key blocks and 128-row tiles, one and two tiles, key slices, windows that
+start inside a block, head sizes that end inside a 64-column chunk, groups that do not fill a tile, and rows nobody may see."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# results are bf16 (2^-9 / sqrt(3) = 1.1e-3 in the 2-norm, at most 2^-8 of a value); probabilities enter as two bf16 terms, 2^-17 each
+EXACT_P = 2e-3
+BF16_P = 1e-2           # D = 128 without a window: probabilities in bf16
+
+
+def _rel(a, b):
+    return ((a.double() - b).norm() / b.norm().clamp_min(1e-30)).item()
+
+
+def _attend(q, k, v, scale, first, window, causal=True):
+    """One sequence in 64 bits: q [n, Hq, D] at positions first.., k, v [m, Hkv, D]."""
+    rep = q.shape[1] // k.shape[1]
+    k, v = k.double().repeat_interleave(rep, 1), v.double().repeat_interleave(rep, 1)
+    s = torch.einsum("qhd,khd->hqk", q.double(), k) * scale
+    at, key = torch.arange(q.shape[0], device=q.device)[:, None] + first, torch.arange(k.shape[0], device=q.device)[None, :]
+    hide = (key > at) if causal else torch.zeros_like(key > at)
+    if window > 0:
+        hide = hide | (key <= at - window)
+    s = s.masked_fill(hide[None], float("-inf"))
+    p = torch.softmax(s, -1).nan_to_num(0.0)
+    return torch.einsum("hqk,khd->qhd", p, v)
+
+
+@pytest.mark.parametrize("hq,hkv,dim,window", [(16, 2, 256, 0), (16, 4, 256, 100), (8, 2, 128, 64), (64, 4, 128, 0), (12, 1, 72, 0), (4, 4, 8, 33), (16, 1, 192, 1000),
+                                               (128, 1, 64, 1)])
+@pytest.mark.parametrize("new,total", [([1], [1]), ([127, 1, 128], [127, 128, 128]), ([129, 257], [129, 300]), ([1, 1, 1], [1, 64, 900]), ([40, 2], [1040, 66]), ([5], [2000])])
+def test_paged(hq, hkv, dim, window, new, total):
+    from nanoengine_b200.ops import sm100, sm100_attn
+    sm100.clear_kernel_status()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    nb = [-(-n // 64) for n in total]
+    bt = torch.full((len(new), max(nb) + 1), -1, dtype=torch.int32, device="cuda")           # a table entry behind the context is no page
+    perm = torch.randperm(sum(nb), generator=g, device="cuda", dtype=torch.int32) + 1
+    kc = torch.full((sum(nb) + 2, 64, hkv, dim), float("nan"), dtype=torch.bfloat16, device="cuda")      # and a row behind it no number
+    vc = kc.clone()
+    q = torch.randn(sum(new), hq, dim, generator=g, device="cuda").to(torch.bfloat16)
+    want, at, o = [], 0, 0
+    for i, (n, m) in enumerate(zip(new, total)):
+        pages = perm[at: at + nb[i]]
+        at += nb[i]
+        bt[i, : nb[i]] = pages
+        k, v = (torch.randn(m, hkv, dim, generator=g, device="cuda").to(torch.bfloat16) for _ in "kv")
+        slots = (pages.long()[:, None] * 64 + torch.arange(64, device="cuda")[None]).flatten()[:m]
+        kc.view(-1, hkv, dim)[slots], vc.view(-1, hkv, dim)[slots] = k, v
+        want.append(_attend(q[o: o + n], k, v, dim ** -0.5, m - n, window))
+        if window > 0 and m - n - window >= 64:            # pages wholly in front of the window may have been given away
+            gone = (m - n - window + 1) // 64
+            vc[pages[:gone].long()] = float("inf")
+        o += n
+    cu = torch.tensor([0] + torch.tensor(new).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    calls = sm100_attn.PROMPT_TC_CALLS[0]
+    if dim == 128 and window == 0 and sum(new) <= len(new):
+        vc, kc = vc.nan_to_num(0.0), kc.nan_to_num(0.0)    # the decode kernel multiplies whole pages
+    got = sm100_attn.gqa_attention_paged(q, kc, vc, bt, cu, torch.tensor(total, dtype=torch.int32, device="cuda"), dim ** -0.5, window)
+    assert sm100.kernel_status()[0] == 0
+    assert (sm100_attn.PROMPT_TC_CALLS[0] > calls) == (not (dim == 128 and window == 0 and sum(new) <= len(new)))
+    assert _rel(got, torch.cat(want)) < (BF16_P if dim == 128 and window == 0 else EXACT_P)
+
+
+@pytest.mark.parametrize("heads,dim", [(16, 72), (3, 80), (2, 256), (1, 64), (5, 136)])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("lens", [[1], [128, 0, 1, 127], [129, 300, 64], [700]])
+def test_ragged(heads, dim, causal, lens):
+    from nanoengine_b200.ops import sm100, sm100_attn
+    sm100.clear_kernel_status()
+    g = torch.Generator(device="cuda").manual_seed(4)
+    t = sum(lens)
+    qkv = torch.randn(t, 3, heads, dim, generator=g, device="cuda").to(torch.bfloat16)         # strided views, as a fused projection leaves them
+    q, k, v = qkv.unbind(1)
+    cu = [0] + torch.tensor(lens).cumsum(0).tolist()
+    want = torch.cat([_attend(q[a:b], k[a:b], v[a:b], dim ** -0.5, 0, 0, causal) for a, b in zip(cu, cu[1:])])
+    calls = sm100_attn.PROMPT_TC_CALLS[0]
+    got = sm100.attention_varlen(q, k, v, torch.tensor(cu, dtype=torch.int32, device="cuda"), dim ** -0.5, causal)
+    assert sm100.kernel_status()[0] == 0 and sm100_attn.PROMPT_TC_CALLS[0] == calls + 1
+    assert _rel(got, want) < EXACT_P
+
+
+def test_a_sequence_does_not_see_its_neighbour_s_infinities():
+    from nanoengine_b200.ops import sm100
+    x = torch.randn(3, 200, 4, 72, device="cuda").to(torch.bfloat16)
+    cu = torch.tensor([0, 100, 200], dtype=torch.int32, device="cuda")
+    clean = sm100.attention_varlen(*x, cu, 0.1)
+    x[:, 100:] = float("inf")
+    assert torch.equal(sm100.attention_varlen(*x, cu, 0.1)[:100], clean[:100])
