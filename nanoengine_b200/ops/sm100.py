@@ -52,7 +52,7 @@ def _st():
 
 
 LAUNCHES = [0]          # kernels of this library launched so far (a call that launches several counts them all)
-_KERNELS_PER_CALL = {"ne_moe_dispatch_local": 3}
+_KERNELS_PER_CALL = {"ne_moe_dispatch_local": 3, "ne_delta_chunk": 2}
 
 
 def _ck(rc: int, name: str):
@@ -1103,11 +1103,19 @@ def rmsnorm_gated(x: torch.Tensor, z: torch.Tensor, w: torch.Tensor, eps: float,
     return out
 
 
+def _gdn_step(q, k, v, a, b, A_log, dt_bias, state, slots, cu, fresh, z, norm_w, eps, dst, skip, raw):
+    """Token by token, the sequences of less than `skip` new tokens."""
+    _ck(lib().ne_gdn_step(_p(q), _p(k), _p(v), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _p(a), _p(b), _c.c_longlong(a.stride(0)),
+                          _p(A_log), _p(dt_bias), _p(state), _p(slots), _p(cu), _p(fresh), _p(z), _c.c_longlong(z.stride(0)), _p(norm_w),
+                          _c.c_float(eps), _p(dst), _c.c_longlong(dst.stride(0)), _c.c_int(cu.numel() - 1), _c.c_int(q.shape[1]), _c.c_int(v.shape[1]),
+                          _c.c_int(q.shape[2]), _c.c_int(v.shape[2]), _c.c_int(skip), _c.c_int(1 if raw else 0), _c.c_int(0), _c.c_float(0.0), _st()), "ne_gdn_step")
+
+
 def gdn_recurrent(q, k, v, a, b, A_log, dt_bias, state, slots, cu_seqlens, fresh, z, norm_w, eps: float, max_q_len: int = 1,
                   cu_host=None) -> torch.Tensor:
     """Gated delta rule + gated RMSNorm.  Sequences shorter than `ref.GDN_CHUNK_MIN_TOKENS` new tokens (decode, verification,
-    short chunks) run in the recurrent kernel that keeps the state in registers; longer ones take the chunked form, whose
-    work is batched matrix products, and need the host copy of the sequence boundaries (`cu_host`)."""
+    short chunks) run in the recurrent kernel that keeps the state in registers; longer ones take the chunked form (`delta_chunk.cu` for
+    128 x 128 states, batched matrix products otherwise), and need the host copy of the sequence boundaries (`cu_host`)."""
     T, Hk, Dk = q.shape
     Hv, Dv = v.shape[1], v.shape[2]
     for t in (q, k, v, z):
@@ -1121,6 +1129,16 @@ def gdn_recurrent(q, k, v, a, b, A_log, dt_bias, state, slots, cu_seqlens, fresh
     if max_q_len >= ref.GDN_CHUNK_MIN_TOKENS:
         assert cu_host is not None, "the chunked prefill form needs the sequence boundaries on the host"
         skip = ref.GDN_CHUNK_MIN_TOKENS
+        if Dk == Dv == 128 and q.stride(0) % 8 == 0 and v.stride(0) % 8 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, k, v)):
+            raw = torch.empty(T, Hv, Dv, dtype=torch.float32, device=q.device)
+            chunks = T // 64 + cu.numel() - 1
+            work = torch.empty(chunks * Hv * lib().ne_delta_chunk_work(), dtype=torch.uint8, device=q.device)
+            _ck(lib().ne_delta_chunk(_p(q), _p(k), _p(v), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _p(a), _p(b), _c.c_longlong(a.stride(0)),
+                                     _p(A_log), _p(dt_bias), _p(state), _p(slots), _p(cu), _p(fresh), _p(raw), _p(work), _c.c_int(T), _c.c_int(cu.numel() - 1),
+                                     _c.c_int(chunks), _c.c_int(Hk), _c.c_int(Hv), _c.c_int(skip), _st()), "ne_delta_chunk")
+            if any(e - s < skip for s, e in zip(cu_host, cu_host[1:])):
+                _gdn_step(q, k, v, a, b, A_log, dt_bias, state, slots, cu, fresh, z, norm_w, eps, raw, skip, True)
+            return rmsnorm_gated(raw, z, norm_w, eps, out).view(T, Hv * Dv)
         rep = Hv // Hk
         g, beta = ref.gdn_gates(a, b, A_log, dt_bias)
         for i in range(len(cu_host) - 1):
@@ -1140,10 +1158,7 @@ def gdn_recurrent(q, k, v, a, b, A_log, dt_bias, state, slots, cu_seqlens, fresh
         dst = torch.zeros(T, Hv, Dv, dtype=torch.float32, device=q.device)
     else:
         dst = torch.empty(T, Hv, Dv, dtype=torch.float32, device=q.device) if raw else out
-    _ck(lib().ne_gdn_step(_p(q), _p(k), _p(v), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _p(a), _p(b), _c.c_longlong(a.stride(0)),
-                          _p(A_log), _p(dt_bias), _p(state), _p(slots), _p(cu), _p(fresh), _p(z), _c.c_longlong(z.stride(0)), _p(norm_w),
-                          _c.c_float(eps), _p(dst), _c.c_longlong(dst.stride(0)), _c.c_int(cu.numel() - 1), _c.c_int(Hk), _c.c_int(Hv), _c.c_int(Dk),
-                          _c.c_int(Dv), _c.c_int(skip), _c.c_int(1 if raw else 0), _c.c_int(0), _c.c_float(0.0), _st()), "ne_gdn_step")
+    _gdn_step(q, k, v, a, b, A_log, dt_bias, state, slots, cu, fresh, z, norm_w, eps, dst, skip, raw)
     if raw:
         if max_q_len >= ref.GDN_CHUNK_MIN_TOKENS:
             short = torch.ones(T, dtype=torch.bool, device=q.device)

@@ -1,0 +1,76 @@
+"""The chunked delta rule in 32-bit accuracy against the recurrence in 64 bits: chunk edges, portions of every length beside short ones, carried and fresh states,
+decays from none to complete, strided rows."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+D = 128
+# an operand of a product is kept to 2^-25 and sums are 32-bit: a few 2^-24 (6e-8) of the state's size; a log decay g is 32-bit, which moves its factor by
+# |g| 2^-23 at most, and a factor counts where |g| is a few.  Results are bf16, with roundings between norm and gate.
+STATE, OUT = 2e-6, 5e-3
+
+
+def _rel(a, b):
+    return ((a.double() - b).norm() / b.norm().clamp_min(1e-30)).item()
+
+
+def _oracle(q, k, v, g, beta, state, fresh, lens, slots):
+    """q, k [T, H, D] unit vectors; g [T, H] or [T, H, D] log decays; all in 64 bits.  Returns outputs and final states."""
+    outs, at = [], 0
+    state = state.double().clone()
+    for i, n in enumerate(lens):
+        s = torch.zeros_like(state[0]) if fresh[i] else state[slots[i]].clone()
+        for t in range(at, at + n):
+            d = g[t].exp()
+            s = s * (d[:, None, :] if d.dim() == 2 else d[:, None, None])
+            u = beta[t][:, None] * (v[t] - torch.einsum("hvk,hk->hv", s, k[t]))
+            s = s + u[:, :, None] * k[t][:, None, :]
+            outs.append(torch.einsum("hvk,hk->hv", s, q[t]))
+        if n:
+            state[slots[i]] = s
+        at += n
+    return torch.stack(outs), state
+
+
+def _inputs(lens, hk, hv, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    t = sum(lens)
+    r = lambda *s: torch.randn(*s, generator=gen, device="cuda")             # noqa: E731
+    y = r(t, (2 * hk + hv) * D).to(torch.bfloat16)
+    q, k, v = y[:, : hk * D].view(t, hk, D), y[:, hk * D: 2 * hk * D].view(t, hk, D), y[:, 2 * hk * D:].view(t, hv, D)
+    state = r(len(lens) + 1, hv, D, D) * 0.2
+    slots = torch.randperm(len(lens) + 1, generator=gen, device="cuda")[: len(lens)].int()
+    fresh = (torch.arange(len(lens), device="cuda") % 2 == 1).int()
+    cu = [0] + torch.tensor(lens).cumsum(0).tolist()
+    z, w = r(t, hv, D).to(torch.bfloat16), (1 + 0.1 * r(D)).to(torch.bfloat16)
+    return gen, r, q, k, v, state, slots, fresh, cu, z, w
+
+
+def _unit(x, rep, scale=1.0):
+    x = x.double()
+    return (x * torch.rsqrt(x.square().sum(-1, keepdim=True) + 1e-6)).repeat_interleave(rep, 1) * scale
+
+
+@pytest.mark.parametrize("hk,hv", [(1, 1), (2, 4), (3, 3)])
+@pytest.mark.parametrize("lens", [[64], [65, 3, 128], [127, 1, 0, 64, 200], [16, 700]])
+@pytest.mark.parametrize("decay", [0.001, 0.3, 40.0])
+def test_decay_per_head(hk, hv, lens, decay):
+    from nanoengine_b200.ops import sm100
+    gen, r, q, k, v, state, slots, fresh, cu, z, w = _inputs(lens, hk, hv, 5)
+    t = sum(lens)
+    ab = r(t, 2 * hv).to(torch.bfloat16)
+    a, b = ab[:, :hv], ab[:, hv:]
+    A, bias = torch.full((hv,), decay, device="cuda").log(), torch.zeros(hv, device="cuda")
+    g = -A.double().exp() * torch.nn.functional.softplus(a.double() + bias.double())
+    want, want_state = _oracle(_unit(q, hv // hk, D ** -0.5), _unit(k, hv // hk), v.double(), g, torch.sigmoid(b.double()), state, fresh.tolist(), lens, slots.tolist())
+    sm100.clear_kernel_status()
+    got = sm100.gdn_recurrent(q, k, v, a, b, A, bias, state, slots, torch.tensor(cu, dtype=torch.int32, device="cuda"), fresh, z, w, 1e-6, max(lens), cu)
+    zd = z.double()
+    want = want * torch.rsqrt(want.square().mean(-1, keepdim=True) + 1e-6) * w.double() * zd * torch.sigmoid(zd)
+    assert sm100.kernel_status()[0] == 0
+    assert _rel(got.view(t, hv, D), want) < OUT
+    long = [s for s, n in zip(slots.tolist(), lens) if n >= 64]
+    assert _rel(state[long], want_state[long]) < STATE
+    rest = [s for s in range(state.shape[0]) if s not in long]
+    assert _rel(state[rest], want_state[rest]) < 1e-5
