@@ -265,6 +265,44 @@ __global__ void __launch_bounds__(256) rmsnorm_gated_kernel(const float* __restr
   }
 }
 
+// The same for D = 128 and rows on 8-byte boundaries: four neighbouring columns a lane, kRows rows a warp whose loads are all under way before the first is
+// used.  Bound by memory (8 bytes a column); 192,000 rows: 71 us with 2-byte accesses and one row a warp, 53 us so (3.7 TB/s).
+constexpr int kNormRows = 4;
+__global__ void __launch_bounds__(256) rmsnorm_gated128_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ z, long long z_ld,
+                                                              const __nv_bfloat16* __restrict__ w, float eps, __nv_bfloat16* __restrict__ out,
+                                                              long long out_ld, long long rows, int heads, int sigmoid_fp32) {
+  pdl_wait(); pdl_trigger();      // dependent launch: nothing above this line touches global memory
+  const long long row0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * kNormRows;
+  const int c = (threadIdx.x & 31) * 4;
+  float4 f[kNormRows];
+  uint2 g[kNormRows];
+#pragma unroll
+  for (int r = 0; r < kNormRows; r++) {
+    const long long row = min(row0 + r, rows - 1), t = row / heads;
+    f[r] = *reinterpret_cast<const float4*>(x + row * 128 + c);
+    g[r] = *reinterpret_cast<const uint2*>(z + t * z_ld + (row - t * heads) * 128 + c);
+  }
+  const uint2 wu = *reinterpret_cast<const uint2*>(w + c);
+  const float2 w0 = unpack_bf16x2(wu.x), w1 = unpack_bf16x2(wu.y);
+  auto round = [](float v) { return __bfloat162float(__float2bfloat16(v)); };
+#pragma unroll
+  for (int r = 0; r < kNormRows; r++) {
+    const long long row = row0 + r, t = row / heads;
+    const float rstd = rsqrtf(warp_sum(f[r].x * f[r].x + f[r].y * f[r].y + f[r].z * f[r].z + f[r].w * f[r].w) / 128.f + eps);
+    if (row >= rows) return;
+    const float2 z0 = unpack_bf16x2(g[r].x), z1 = unpack_bf16x2(g[r].y);
+    uint2 y;
+    if (sigmoid_fp32) {
+      y.x = pack_bf16x2(f[r].x * rstd * w0.x / (1.f + __expf(-z0.x)), f[r].y * rstd * w0.y / (1.f + __expf(-z0.y)));
+      y.y = pack_bf16x2(f[r].z * rstd * w1.x / (1.f + __expf(-z1.x)), f[r].w * rstd * w1.y / (1.f + __expf(-z1.y)));
+    } else {
+      y.x = pack_bf16x2(round(w0.x * round(f[r].x * rstd)) * round(silu_f(z0.x)), round(w0.y * round(f[r].y * rstd)) * round(silu_f(z0.y)));
+      y.y = pack_bf16x2(round(w1.x * round(f[r].z * rstd)) * round(silu_f(z1.x)), round(w1.y * round(f[r].w * rstd)) * round(silu_f(z1.y)));
+    }
+    *reinterpret_cast<uint2*>(out + t * out_ld + (row - t * heads) * 128 + c) = y;
+  }
+}
+
 // out = o * sigmoid(gate); o, out [T, heads, D] contiguous, gate a strided view (row and head strides in elements); two columns per thread
 __global__ void __launch_bounds__(256) sigmoid_gate_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ gate, long long g_row,
                                                           long long g_head, __nv_bfloat16* __restrict__ out, long long pairs, int heads, int D) {
@@ -338,6 +376,9 @@ extern "C" int ne_rmsnorm_gated(const float* x, const void* z, long long z_ld, c
                                 int heads, int D, int sigmoid_fp32, cudaStream_t st) {
   long long rows = tokens * heads;
   if (rows <= 0) return 0;
+  if (D == 128 && z_ld % 4 == 0 && out_ld % 4 == 0 && ((uintptr_t)x & 15) == 0 && (((uintptr_t)z | (uintptr_t)w | (uintptr_t)out) & 7) == 0)
+    return (int)launch_pdl(rmsnorm_gated128_kernel, dim3((unsigned)((rows + 8 * kNormRows - 1) / (8 * kNormRows))), dim3(256), 0, st, x, (const __nv_bfloat16*)z, z_ld,
+                           (const __nv_bfloat16*)w, eps, (__nv_bfloat16*)out, out_ld, rows, heads, sigmoid_fp32);
   return (int)launch_pdl(rmsnorm_gated_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, st, x, (const __nv_bfloat16*)z, z_ld, (const __nv_bfloat16*)w, eps, (__nv_bfloat16*)out,
                                                                   out_ld, rows, heads, D, sigmoid_fp32);
 }
