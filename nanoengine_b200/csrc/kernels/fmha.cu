@@ -299,8 +299,10 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int j = 0; j < 128; j++) mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(r[j]));
-      // the reference is a whole power of two: rescaling by it is exact, and a probability rounds alike whatever the blocks are
-      const float m_tile = ceilf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * a.scale_log2);
+      float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * a.scale_log2;
+      // 32-bit probabilities: the reference is a whole power of two, so rescaling by it is exact and the two terms of a probability are the same whatever the
+      // slices and blocks are.  bf16 probabilities: the largest one is exactly 1, and a row that looks at few keys has the smaller error.
+      if (kSplitP) m_tile = ceilf(m_tile);
       // lazy rescaling: the reference maximum only moves when the block's maximum exceeds it by more than 2^8
       const bool first_valid = m_run == -INFINITY;
       const float m_new = (first_valid || m_tile > m_run + 8.f) ? fmaxf(m_run, m_tile) : m_run;
@@ -428,15 +430,6 @@ static int fmha_launch(const CUtensorMap& q, const CUtensorMap& k, const CUtenso
 
 using namespace ne;
 
-// Query tokens per CTA tile set (0: sizes this kernel does not cover).  rows: new tokens of the longest sequence, where known (0: unknown).
-extern "C" int ne_fmha_plan(int g, int D, int Dv, int rows, int* tiles) {
-  if (g < 1 || g > 128 || D < 8 || D > 256 || D % 8 || Dv < 8 || Dv > 256 || Dv % 8) return 0;
-  const int tq = 128 / g;
-  // two tiles: one's softmax runs beside the other's products; TMEM holds two accumulators of up to 128 columns, shared memory two Q tiles of up to 192
-  *tiles = Dv <= 128 && D <= 192 && (rows == 0 || rows > tq) ? 2 : 1;
-  return tq * *tiles;
-}
-
 // q [T, Hq, D] with row stride q_ld (elements; heads D apart), keys / values either pages k, v [num_blocks, 64, Hkv, D or Dv] contiguous (block_tables
 // not null) or rows [T, Hkv, D or Dv] with row strides k_ld, v_ld; k_rope not null (ragged only): the last D - Dk_nope columns of every head's key are the
 // row k_rope [T, D - Dk_nope] (row stride r_ld), k_nope heads k_head apart.  context_lens null: keys are the sequence's own tokens.
@@ -447,8 +440,7 @@ extern "C" int ne_fmha(const void* q, long long q_ld, const void* k, long long k
                        float* lse2, cudaStream_t st) {
   if (T <= 0) return 0;
   if (Hkv < 1 || Hq % Hkv || splits < 1 || (splits > 1 && (!part || !lse2)) || grid_x < 1 || Hkv > 65535) return 1001;
-  int most = 0;
-  if (!ne_fmha_plan(Hq / Hkv, D, Dv, 0, &most) || tiles < 1 || tiles > most) return 1002;
+  if (Hq / Hkv > 128 || D < 8 || D > 256 || D % 8 || Dv < 8 || Dv > 256 || Dv % 8 || tiles < 1 || tiles > (Dv <= 128 && D <= 192 ? 2 : 1)) return 1002;
   if (q_ld % 8 || q_ld < (long long)Hq * D || (block_tables == nullptr && (k_ld % 8 || v_ld % 8)) || (k_rope && (block_tables || r_ld % 8 || k_dim % 64 || k_dim >= D))) return 1003;
   FmArgs a;
   a.g = Hq / Hkv; a.tq = 128 / a.g; a.tiles = tiles; a.splits = splits; a.T = T; a.Hq = Hq;

@@ -165,17 +165,33 @@ def mla_attention_paged(q, cache, block_tables, cu_seqlens_q, context_lens, scal
 PROMPT_TC_CALLS = [0]        # launches of the tensor-core prompt attention kernel
 
 
+_FMHA = []
+
+
+def _fmha_call():
+    """The kernel's entry with declared arguments: plain integers cost a fraction of wrapped ones, and short prompts are the host's time."""
+    if not _FMHA:
+        f, i, p, n = _k.lib().ne_fmha, _c.c_int, _c.c_void_p, _c.c_longlong
+        f.argtypes = [p, n, p, n, i, p, n, p, n, i, p, i, p, p, i, i, i, i, i, i, i, i, i, i, i, _c.c_float, i, p, p, p, p]
+        _FMHA.append(f)
+    return _FMHA[0]
+
+
+def _fmha_covers(group: int, D: int, Dv: int) -> bool:
+    return 1 <= group <= 128 and 8 <= D <= 256 and D % 8 == 0 and 8 <= Dv <= 256 and Dv % 8 == 0
+
+
 def _fmha(q, k, v, cu, scale, causal, split_p, block_tables=None, context_lens=None, window=0, k_rope=None, one_token=False):
-    """The tcgen05 prompt kernel; shapes checked by the caller.  Returns None for sizes it does not cover."""
+    """The tcgen05 prompt kernel, for sizes that `_fmha_covers`; rows and pages as the kernel's entry wants them."""
     T, Hq, D = q.shape
     paged = block_tables is not None
     Hkv, Dv = (k.shape[2], v.shape[3]) if paged else (k.shape[1], v.shape[2])
     B = cu.numel() - 1
-    lib = _k.lib()
-    tiles = _c.c_int(0)
-    rows = lib.ne_fmha_plan(_c.c_int(Hq // Hkv), _c.c_int(D), _c.c_int(Dv), _c.c_int(1 if one_token else 0), _c.byref(tiles))
-    if not rows:
-        return None
+    tq = 128 // (Hq // Hkv)
+    # two tiles per CTA: one's softmax runs beside the other's products; TMEM holds two accumulators of up to 128 columns, shared memory two Q tiles of up to
+    # 192.  One tile where pairs would leave SMs idle (and where a sequence has only one).
+    tiles = 1 if one_token or Dv > 128 or D > 192 or min(T, T // (2 * tq) + B) * Hkv < _sms() else 2
+    rows = tq * tiles
     grid = min(T, T // rows + B)
     S = 1
     if paged and grid * Hkv < _sms() // 2:             # few CTAs (small decode batches, short prompts): slice the keys, blocks of 128
@@ -186,14 +202,14 @@ def _fmha(q, k, v, cu, scale, causal, split_p, block_tables=None, context_lens=N
     if S > 1:
         part = torch.empty(S, T, Hq, Dv, dtype=torch.float32, device=q.device)
         lse2 = torch.empty(S, T, Hq, dtype=torch.float32, device=q.device)
-    _k._ck(lib.ne_fmha(_k._p(q), _c.c_longlong(q.stride(0)), _k._p(k), _c.c_longlong(k.stride(0)), _c.c_int(k.shape[-1]), _k._p(k_rope),
-                       _c.c_longlong(0 if k_rope is None else k_rope.stride(0)), _k._p(v), _c.c_longlong(v.stride(0)), _c.c_int(k.shape[0]), _k._p(block_tables),
-                       _c.c_int(block_tables.stride(0) if paged else 0), _k._p(cu), _k._p(context_lens), _c.c_int(B), _c.c_int(T), _c.c_int(Hq), _c.c_int(Hkv),
-                       _c.c_int(D), _c.c_int(Dv), tiles, _c.c_int(grid), _c.c_int(S), _c.c_int(max(0, int(window))), _c.c_int(1 if causal else 0), _c.c_float(scale),
-                       _c.c_int(1 if split_p else 0), _k._p(out), _k._p(part), _k._p(lse2), _k._st()), "ne_fmha")
+    at = lambda t: 0 if t is None else t.data_ptr()          # noqa: E731
+    _k._ck(_fmha_call()(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), k.shape[-1], at(k_rope), 0 if k_rope is None else k_rope.stride(0), v.data_ptr(),
+                        v.stride(0), k.shape[0], at(block_tables), block_tables.stride(0) if paged else 0, cu.data_ptr(), at(context_lens), B, T, Hq, Hkv, D, Dv,
+                        tiles, grid, S, max(0, int(window)), 1 if causal else 0, scale, 1 if split_p else 0, out.data_ptr(), at(part), at(lse2),
+                        torch.cuda.current_stream().cuda_stream), "ne_fmha")
     PROMPT_TC_CALLS[0] += 1
     if S > 1:
-        _k._ck(lib.ne_attn_merge(_k._p(part), _k._p(lse2), _k._p(out), _c.c_int(S), _c.c_longlong(T * Hq), _c.c_int(Dv), _c.c_int(Dv), _k._st()),
+        _k._ck(_k.lib().ne_attn_merge(_k._p(part), _k._p(lse2), _k._p(out), _c.c_int(S), _c.c_longlong(T * Hq), _c.c_int(Dv), _c.c_int(Dv), _k._st()),
                "ne_attn_merge")
     return out
 
@@ -211,9 +227,8 @@ def gqa_attention_paged(q, k_cache, v_cache, block_tables, cu_seqlens_q, context
     lib = _k.lib()
     bt, cu, cl = _i32(block_tables), _i32(cu_seqlens_q), _i32(context_lens)
     q = q if (q.dtype == torch.bfloat16 and q.stride(-1) == 1) else q.to(torch.bfloat16).contiguous()
-    out = torch.empty(T, Hq, D, dtype=torch.bfloat16, device=q.device)
     if T == 0:
-        return out
+        return torch.empty(T, Hq, D, dtype=torch.bfloat16, device=q.device)
     group = Hq // Hkv
     B = cl.numel()
     pages64 = (k_cache.dtype == torch.bfloat16 and v_cache.dtype == torch.bfloat16 and k_cache.shape[1] == 64 and Hq % Hkv == 0 and group <= 128
@@ -221,9 +236,8 @@ def gqa_attention_paged(q, k_cache, v_cache, block_tables, cu_seqlens_q, context
     if D == 128 and window <= 0 and pages64 and group & (group - 1) == 0:
         q = q.contiguous()
         if T > B:                                      # some sequence has more than one new token
-            got = _fmha(q, k_cache, v_cache, cu, scale, True, False, bt, cl)
-            if got is not None:
-                return got
+            return _fmha(q, k_cache, v_cache, cu, scale, True, False, bt, cl)
+        out = torch.empty(T, Hq, D, dtype=torch.bfloat16, device=q.device)
         # tcgen05 kernel: one CTA per (kv head, tile of 128 (token, head) rows, key slice)
         tq = 128 // group
         max_tiles = min(T, T // tq + B)
@@ -242,10 +256,10 @@ def gqa_attention_paged(q, k_cache, v_cache, block_tables, cu_seqlens_q, context
                    "ne_attn_merge")
         return out
     assert group % 4 == 0 or group == 1 and Hq % 4 == 0 or Hkv == Hq, "query heads per kv head must be a multiple of 4"
-    if pages64 and scale > 0 and k_cache.shape[3] == v_cache.shape[3] == D and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0 and D % 8 == 0:
-        got = _fmha(q if _rows16(q) else q.clone(memory_format=torch.contiguous_format), k_cache, v_cache, cu, scale, True, True, bt, cl, window, one_token=T <= B)
-        if got is not None:
-            return got
+    if (pages64 and scale > 0 and _fmha_covers(group, D, D) and k_cache.shape[3] == v_cache.shape[3] == D and k_cache.data_ptr() % 16 == 0
+            and v_cache.data_ptr() % 16 == 0):
+        return _fmha(q if _rows16(q) else q.clone(memory_format=torch.contiguous_format), k_cache, v_cache, cu, scale, True, True, bt, cl, window, one_token=T <= B)
+    out = torch.empty(T, Hq, D, dtype=torch.bfloat16, device=q.device)
     _k._ck(lib.ne_attn_generic(_k._p(q), _c.c_longlong(q.stride(0)), _c.c_int(q.stride(1)), _k._p(k_cache), _k._p(v_cache),
                                _c.c_longlong(Hkv * D), _c.c_int(D), _c.c_int(group), _k._p(bt), _c.c_int(bt.stride(0)), _c.c_int(k_cache.shape[1]),
                                _k._p(cu), _k._p(cl), _c.c_int(cl.numel()), _k._p(None), _c.c_int(0), _k._p(out), _c.c_longlong(Hq * D), _c.c_int(D),
@@ -375,10 +389,8 @@ def attention_varlen(q, k, v, cu_seqlens, scale, causal: bool = False):
     if T == 0:
         return torch.empty(T, H, D, dtype=torch.bfloat16, device=q.device)
     cu = _i32(cu_seqlens)
-    if scale > 0 and D % 8 == 0 and D <= 256 and k.shape == q.shape and v.shape == q.shape:
-        got = _fmha(*[t if _rows16(t) else t.clone(memory_format=torch.contiguous_format) for t in (q, k, v)], cu, scale, causal, True)
-        if got is not None:
-            return got
+    if scale > 0 and _fmha_covers(1, D, D) and k.shape == q.shape and v.shape == q.shape:
+        return _fmha(*[t if _rows16(t) else t.clone(memory_format=torch.contiguous_format) for t in (q, k, v)], cu, scale, causal, True)
     k, v = k.contiguous(), v.contiguous()
     out = torch.empty(T, H, D, dtype=torch.bfloat16, device=q.device)
     lens = (cu[1:] - cu[:-1])
