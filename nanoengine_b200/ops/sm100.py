@@ -1103,6 +1103,25 @@ def rmsnorm_gated(x: torch.Tensor, z: torch.Tensor, w: torch.Tensor, eps: float,
     return out
 
 
+def _delta_groups(q, k, v, g, b, A_log, dt_bias, lower_bound, state, slots, cu, fresh, raw, max_n, per_channel):
+    """Four tokens at a time, 128 x 128 states, the sequences of less than `max_n` new tokens."""
+    _ck(lib().ne_delta_groups(_p(q), _p(k), _p(v), _p(g), _p(b), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _c.c_longlong(g.stride(0)),
+                              _c.c_longlong(b.stride(0)), _p(A_log), _p(dt_bias), _c.c_float(lower_bound), _p(state), _p(slots), _p(cu), _p(fresh), _p(raw),
+                              _c.c_int(cu.numel() - 1), _c.c_int(q.shape[1]), _c.c_int(v.shape[1]), _c.c_int(max_n), _c.c_int(1 if per_channel else 0), _st()),
+        "ne_delta_groups")
+
+
+def _delta_rows16(q, k, v, state):
+    """128 x 128 states with rows that the prompt kernels of the delta rule can copy in 16-byte pieces."""
+    return (q.shape[2] == v.shape[2] == 128 and q.stride(0) % 8 == 0 and k.stride(0) == q.stride(0) and v.stride(0) % 8 == 0
+            and all(t.data_ptr() % 16 == 0 for t in (q, k, v, state)))
+
+
+# Mean portion (tokens) above which four tokens at a time beat one at a time: us for one / four, 32 heads: 64 portions of 2: 72 / 92, 4 of 8: 52 / 53 (both
+# the host's), 16 of 16: 106 / 53, 11 of 55 (16 heads): 153 / 66, 16 of 370: 2208 / 724
+GROUPS_MIN_MEAN = 4
+
+
 def _gdn_step(q, k, v, a, b, A_log, dt_bias, state, slots, cu, fresh, z, norm_w, eps, dst, skip, raw):
     """Token by token, the sequences of less than `skip` new tokens."""
     _ck(lib().ne_gdn_step(_p(q), _p(k), _p(v), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _p(a), _p(b), _c.c_longlong(a.stride(0)),
@@ -1129,14 +1148,17 @@ def gdn_recurrent(q, k, v, a, b, A_log, dt_bias, state, slots, cu_seqlens, fresh
     if max_q_len >= ref.GDN_CHUNK_MIN_TOKENS:
         assert cu_host is not None, "the chunked prefill form needs the sequence boundaries on the host"
         skip = ref.GDN_CHUNK_MIN_TOKENS
-        if Dk == Dv == 128 and q.stride(0) % 8 == 0 and v.stride(0) % 8 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, k, v)):
+        if _delta_rows16(q, k, v, state):
             raw = torch.empty(T, Hv, Dv, dtype=torch.float32, device=q.device)
             chunks = T // 64 + cu.numel() - 1
             work = torch.empty(chunks * Hv * lib().ne_delta_chunk_work(), dtype=torch.uint8, device=q.device)
             _ck(lib().ne_delta_chunk(_p(q), _p(k), _p(v), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _p(a), _p(b), _c.c_longlong(a.stride(0)),
                                      _p(A_log), _p(dt_bias), _p(state), _p(slots), _p(cu), _p(fresh), _p(raw), _p(work), _c.c_int(T), _c.c_int(cu.numel() - 1),
                                      _c.c_int(chunks), _c.c_int(Hk), _c.c_int(Hv), _c.c_int(skip), _st()), "ne_delta_chunk")
-            if any(e - s < skip for s, e in zip(cu_host, cu_host[1:])):
+            short = [e - s for s, e in zip(cu_host, cu_host[1:]) if e - s < skip]
+            if sum(short) > GROUPS_MIN_MEAN * len(short):
+                _delta_groups(q, k, v, a, b, A_log, dt_bias, 0.0, state, slots, cu, fresh, raw, skip, False)
+            elif short:
                 _gdn_step(q, k, v, a, b, A_log, dt_bias, state, slots, cu, fresh, z, norm_w, eps, raw, skip, True)
             return rmsnorm_gated(raw, z, norm_w, eps, out).view(T, Hv * Dv)
         rep = Hv // Hk
@@ -1152,6 +1174,10 @@ def gdn_recurrent(q, k, v, a, b, A_log, dt_bias, state, slots, cu_seqlens, fresh
             o, S = ref.gdn_chunked(qn, kn, v[s:e].float(), g[s:e], beta[s:e], S0)
             state.index_copy_(0, sl, S[None])
             rmsnorm_gated(o, z[s:e], norm_w, eps, out[s:e])
+    elif T > GROUPS_MIN_MEAN * (cu.numel() - 1) and _delta_rows16(q, k, v, state):
+        raw = torch.empty(T, Hv, Dv, dtype=torch.float32, device=q.device)
+        _delta_groups(q, k, v, a, b, A_log, dt_bias, 0.0, state, slots, cu, fresh, raw, skip, False)
+        return rmsnorm_gated(raw, z, norm_w, eps, out).view(T, Hv * Dv)
     raw = bool(lib().ne_gdn_step_raw_only(_c.c_int(Dk), _c.c_int(Dv)))     # large states: several CTAs per head, norm in its own kernel
     if raw and max_q_len >= ref.GDN_CHUNK_MIN_TOKENS:
         # rows of the long sequences were already normalised into `out`; the recurrent kernel's raw rows go to their own buffer
@@ -1294,8 +1320,8 @@ def general_delta(proj: torch.Tensor, decay: torch.Tensor, w0: torch.Tensor, a_b
 
 
 def kda_recurrent(q, k, v, raw_g, b, A_log, dt_bias, lower_bound, state, slots, cu_seqlens, fresh, gate, norm_w, eps: float) -> torch.Tensor:
-    """Kimi delta attention: the delta rule with a log-decay per key channel, then the sigmoid-gated RMSNorm.  Every sequence,
-    prompt chunks included, runs token by token in the kernel that keeps the 128 x 128 state in registers."""
+    """Kimi delta attention: the delta rule with a log-decay per key channel, then the sigmoid-gated RMSNorm.  The 128 x 128 state stays in registers; decode
+    steps run token by token (gdn.cu), longer portions four tokens at a time (delta_groups.cu)."""
     T, H, Dk = q.shape
     Dv = v.shape[2]
     assert Dk == 128 and Dv == 128 and k.shape == q.shape and v.shape[1] == H, "the CUDA form covers 128 x 128 states"
@@ -1307,11 +1333,15 @@ def kda_recurrent(q, k, v, raw_g, b, A_log, dt_bias, lower_bound, state, slots, 
     assert A_log.dtype == torch.float32 and dt_bias.dtype == torch.float32 and dt_bias.numel() == H * Dk and norm_w.dtype == torch.bfloat16
     slots, cu, fresh = _i32(slots), _i32(cu_seqlens), _i32(fresh)
     raw = torch.empty(T, H, Dv, dtype=torch.float32, device=q.device)
-    _ck(lib().ne_gdn_step(_p(q), _p(k), _p(v), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _p(raw_g), _p(b), _c.c_longlong(b.stride(0)),
-                          _p(A_log), _p(dt_bias), _p(state), _p(slots), _p(cu), _p(fresh), _p(gate), _c.c_longlong(gate.stride(0)), _p(norm_w),
-                          _c.c_float(eps), _p(raw), _c.c_longlong(raw.stride(0)), _c.c_int(cu.numel() - 1), _c.c_int(H), _c.c_int(H), _c.c_int(Dk),
-                          _c.c_int(Dv), _c.c_int(1 << 30), _c.c_int(1), _c.c_int(1), _c.c_float(float(lower_bound) if lower_bound is not None else 0.0),
-                          _st()), "ne_gdn_step")
+    lb = float(lower_bound) if lower_bound is not None else 0.0
+    if T > GROUPS_MIN_MEAN * (cu.numel() - 1) and _delta_rows16(q, k, v, state) and raw_g.data_ptr() % 16 == 0:
+        _delta_groups(q, k, v, raw_g, b, A_log, dt_bias, lb, state, slots, cu, fresh, raw, 1 << 30, True)
+    else:
+        _ck(lib().ne_gdn_step(_p(q), _p(k), _p(v), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _p(raw_g), _p(b), _c.c_longlong(b.stride(0)),
+                              _p(A_log), _p(dt_bias), _p(state), _p(slots), _p(cu), _p(fresh), _p(gate), _c.c_longlong(gate.stride(0)), _p(norm_w),
+                              _c.c_float(eps), _p(raw), _c.c_longlong(raw.stride(0)), _c.c_int(cu.numel() - 1), _c.c_int(H), _c.c_int(H), _c.c_int(Dk),
+                              _c.c_int(Dv), _c.c_int(1 << 30), _c.c_int(1), _c.c_int(1), _c.c_float(lb),
+                              _st()), "ne_gdn_step")
     w = norm_w.expand(Dv) if norm_w.numel() == Dv else norm_w
     return rmsnorm_gated(raw, gate, w.contiguous(), eps, sigmoid=True).view(T, H * Dv)
 

@@ -1,4 +1,4 @@
-"""The chunked delta rule in 32-bit accuracy against the recurrence in 64 bits: chunk edges, portions of every length beside short ones, carried and fresh states,
+"""The delta rule over prompts, chunked or in groups of four tokens, in 32-bit, against the recurrence in 64 bits: chunk edges, portions of every length beside short ones, carried and fresh states,
 decays from none to complete, strided rows."""
 import pytest
 import torch
@@ -53,7 +53,7 @@ def _unit(x, rep, scale=1.0):
 
 
 @pytest.mark.parametrize("hk,hv", [(1, 1), (2, 4), (3, 3)])
-@pytest.mark.parametrize("lens", [[64], [65, 3, 128], [127, 1, 0, 64, 200], [16, 700]])
+@pytest.mark.parametrize("lens", [[64], [65, 3, 128], [127, 1, 0, 64, 200], [16, 700], [63, 5, 17, 16]])
 @pytest.mark.parametrize("decay", [0.001, 0.3, 40.0])
 def test_decay_per_head(hk, hv, lens, decay):
     from nanoengine_b200.ops import sm100
@@ -70,7 +70,27 @@ def test_decay_per_head(hk, hv, lens, decay):
     want = want * torch.rsqrt(want.square().mean(-1, keepdim=True) + 1e-6) * w.double() * zd * torch.sigmoid(zd)
     assert sm100.kernel_status()[0] == 0
     assert _rel(got.view(t, hv, D), want) < OUT
-    long = [s for s, n in zip(slots.tolist(), lens) if n >= 64]
+    long = [s for s, n in zip(slots.tolist(), lens) if n >= 64 or min(lens) > 4]         # the others one token at a time
     assert _rel(state[long], want_state[long]) < STATE
     rest = [s for s in range(state.shape[0]) if s not in long]
     assert _rel(state[rest], want_state[rest]) < 1e-5
+
+
+@pytest.mark.parametrize("heads", [1, 3])
+@pytest.mark.parametrize("lens", [[5], [16, 17, 1, 0, 33], [1, 300], [15, 48] * 40])
+@pytest.mark.parametrize("bound,scale", [(-5.0, 0.5), (None, 0.05), (-0.01, 1.0), (None, 30.0)])
+def test_decay_per_channel(heads, lens, bound, scale):
+    from nanoengine_b200.ops import sm100
+    gen, r, q, k, v, state, slots, fresh, cu, z, w = _inputs(lens, heads, heads, 6)
+    t = sum(lens)
+    a, b = r(t, heads * D).to(torch.bfloat16), r(t, heads).to(torch.bfloat16)
+    A, bias = torch.full((heads,), scale, device="cuda").log(), r(heads * D)
+    x = a.double().view(t, heads, D) + bias.double().view(1, heads, D)
+    e = A.double().exp()[None, :, None]
+    g = bound * torch.sigmoid(e * x) if bound is not None else -e * torch.nn.functional.softplus(x)
+    want, want_state = _oracle(_unit(q, 1, D ** -0.5), _unit(k, 1), v.double(), g, torch.sigmoid(b.double()), state, fresh.tolist(), lens, slots.tolist())
+    sm100.clear_kernel_status()
+    got = sm100.kda_recurrent(q, k, v, a, b, A, bias, bound, state, slots, torch.tensor(cu, dtype=torch.int32, device="cuda"), fresh, z, w, 1e-6)
+    want = want * torch.rsqrt(want.square().mean(-1, keepdim=True) + 1e-6) * w.double() * torch.sigmoid(z.double())
+    assert sm100.kernel_status()[0] == 0
+    assert _rel(got.view(t, heads, D), want) < OUT and _rel(state, want_state) < STATE
