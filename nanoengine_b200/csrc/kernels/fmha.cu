@@ -2,19 +2,20 @@
 // multiples of 8 (queries / keys and values may differ), any group of query heads per key / value head up to 128, causal or not, a window of the
 // last keys; keys and values in 64-token cache pages, or as rows of the same ragged tokens (vision encoders, prompts without a cached prefix).
 //
-// One CTA = one KV head x up to two tiles of 128 (token, head of the group) rows of ONE sequence x one slice of its keys, in blocks of 128 keys.
-// Work items n = (block, tile) go through two TMEM score slots of 128 columns:
-//     S(n) = Q K^T        (tcgen05.mma kind::f16, M = 128, N = 128: with N = 64 the operand reads from shared memory would take longer than the
-//                          products; K = 16 steps up to the head size, so a head of 72 pays for 80)
-//     P(n) = exp2(S - m)  one warpgroup per tile; bf16 pairs written over S(n) in TMEM, the A operand of the second product
-//     O(t) += P(n) V      (N = head size up to the next multiple of 16; V read MN-major)
-// While one tile's softmax runs, the other tile's products do.  The products of a tile are issued by one thread in the order S, then PV(n) S(n+2) ..:
-// they complete in order, so S(n+2) may overwrite P(n) without a barrier.  Each tile has an issuer of its own: a barrier test costs the thread 300 cycles
-// once products are queued before it, and one issuer for both tiles was what bounded the kernel (4800 cycles for two 128 x 128 x 128 items, of which 2048
-// are products).  With a single tile (short sequences, value heads above 128 columns) the two slots are its consecutive key blocks.
+// One CTA = one KV head x up to two tiles of 128 (token, head of the group) rows of ONE sequence x one slice of its keys, in blocks of 64 keys (a page).
+// Every tile t has two TMEM score slots of 64 columns, block j in slot j & 1, and a thread that issues its products in the order S(0) S(1), then
+// PV(j) S(j+2) ..:
+//     S(j) = Q K^T        (tcgen05.mma kind::f16, M = 128, N = 64, K = 16 steps up to the head size, so a head of 72 pays for 80)
+//     P(j) = exp2(S - m)  one warpgroup per tile; bf16 pairs written over S(j) in TMEM, the A operand of the second product
+//     O   += P(j) V       (N = head size up to the next multiple of 16; V read MN-major)
+// They complete in order, so S(j+2) may overwrite P(j) without a barrier, and the softmax finds S(j+1) ready when it has handed P(j) on.  (Blocks of 128
+// keys with one slot a tile read less shared memory per product, but then scores, softmax and products of a tile are one chain: 4150 cycles for 128 keys of
+// two tiles, whether one or two warpgroups share a tile's softmax; so it is 3900.  One tile per CTA and two CTAs per SM, or an issuer each for scores and
+// products, were no faster.)
+// A barrier test costs an issuing thread 300 cycles once products are queued before it, hence an issuer per tile, and tests in threes.
 // kSplitP: probabilities stay 32-bit in effect: bf16 head and bf16 remainder (2^-17), two products against V.  Taken where the plain kernel this one
 // replaced kept them in fp32.
-// Shared memory: Q, then a ring of 16 KB slots (128 keys x 64 columns) shared by K and V, loaded in the order of first use; the chunks of a block's K
+// Shared memory: Q, then a ring of 8 KB slots (64 keys x 64 columns) shared by K and V, loaded in the order of first use; the chunks of a block's K
 // or V (a group) share one barrier.
 // Rows of V in front of the window or past the last visible key (pages that belong to nobody, rows of the next sequence) are zeroed in shared
 // memory before their product: 0 x inf there would reach the result.  Warp 0: TMA producer, 1 and 2: MMA issuers of tile 0 and 1, 3: that zeroing,
@@ -26,10 +27,11 @@
 namespace ne {
 
 constexpr int kKernelFm = 27;
-constexpr int kFmBlk = 128;                    // keys per block
-constexpr int kFmSlot = kFmBlk * 128;          // 128 rows x 64 bf16 columns
-constexpr int kFmMaxSlots = 12;
-constexpr int kFmGroups = 16;                  // barriers of groups in flight; a group has at least one slot
+constexpr int kFmBlk = 64;                     // keys per block: one cache page
+constexpr int kFmSlot = kFmBlk * 128;          // 64 rows x 64 bf16 columns
+constexpr int kFmQ = 128 * 128;                // a chunk of Q: 128 rows x 64 columns
+constexpr int kFmMaxSlots = 24;
+constexpr int kFmGroups = 32;                  // barriers of groups in flight; a group has at least one slot
 
 struct FmArgs {
   const int* block_tables; int bt_stride;      // paged
@@ -56,6 +58,14 @@ __device__ __forceinline__ uint32_t ex2(uint32_t x) {
   return x;
 }
 
+__device__ __forceinline__ void mbar_test3(uint32_t a, uint32_t pa, uint32_t b, uint32_t pb, uint32_t c, uint32_t pc, bool& ra, bool& rb, bool& rc) {
+  uint32_t x, y, z;
+  asm volatile("{\n .reg .pred p, q, r;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%3], %4;\n mbarrier.test_wait.parity.shared::cta.b64 q, [%5], %6;\n"
+               " mbarrier.test_wait.parity.shared::cta.b64 r, [%7], %8;\n selp.u32 %0, 1, 0, p;\n selp.u32 %1, 1, 0, q;\n selp.u32 %2, 1, 0, r;\n}\n"
+               : "=r"(x), "=r"(y), "=r"(z) : "r"(a), "r"(pa), "r"(b), "r"(pb), "r"(c), "r"(pc) : "memory");
+  ra = x; rb = y; rc = z;
+}
+
 // kWG: softmax warpgroups = most tiles per CTA
 template <int kWG, bool kSplitP>
 __global__ void __launch_bounds__(128 + 128 * kWG, 1)
@@ -66,13 +76,14 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
   // swizzled tiles need 1024-byte alignment; behind static shared memory the dynamic part starts on a 16-byte boundary
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;                                    // [tile][chunk][128 rows x 128 B]
-  uint8_t* sKV = sQ + kWG * a.nc * kFmSlot;
-  __shared__ uint64_t bars[2 * kFmGroups + 19];
+  uint8_t* sKV = sQ + kWG * a.nc * kFmQ;
+  __shared__ uint64_t bars[2 * kFmGroups + 17];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort, s_seq, s_tok;
   volatile int* abort_flag = &s_abort;
-  const uint32_t b_full = smem_u32(bars), b_empty = b_full + 8 * kFmGroups, b_q = b_empty + 8 * kFmGroups, b_s = b_q + 8, b_p = b_s + 16, b_pv = b_p + 16,
-                 b_go = b_pv + 16, b_fix = b_go + 16, b_turn = b_fix + 16;
+  // scores, probabilities, products: [tile][block & 1]
+  const uint32_t b_full = smem_u32(bars), b_empty = b_full + 8 * kFmGroups, b_q = b_empty + 8 * kFmGroups, b_s = b_q + 8, b_p = b_s + 32, b_pv = b_p + 32,
+                 b_go = b_pv + 32, b_fix = b_go + 16;
   const int warp = threadIdx.x >> 5;
   const int hkv = blockIdx.y, split = blockIdx.z;
   if (warp == 0) {
@@ -100,14 +111,11 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
     blk0 = first + split * per_split;
     nblk = max(0, min(total, (split + 1) * per_split) - split * per_split);
   }
-  const int items = nblk * nt;
   if (threadIdx.x == 32) {
     for (int i = 0; i < kFmGroups; i++) { mbar_init(b_full + 8 * i, 1); mbar_init(b_empty + 8 * i, nt); }
     mbar_init(b_q, 1);
-    for (int i = 0; i < 2; i++) {
-      mbar_init(b_s + 8 * i, 1); mbar_init(b_p + 8 * i, 4); mbar_init(b_pv + 8 * i, 1); mbar_init(b_go + 8 * i, 1); mbar_init(b_fix + 8 * i, 32);
-    }
-    for (int i = 0; i < 8; i++) mbar_init(b_turn + 8 * i, 1);
+    for (int i = 0; i < 4; i++) { mbar_init(b_s + 8 * i, 1); mbar_init(b_p + 8 * i, 4); mbar_init(b_pv + 8 * i, 1); }
+    for (int i = 0; i < 2; i++) { mbar_init(b_go + 8 * i, 1); mbar_init(b_fix + 8 * i, 32); }
     s_abort = 0;
     mbar_fence_init();
   }
@@ -115,26 +123,24 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   pdl_trigger();                  // behind the TMEM allocation: a CTA of the next grid never holds columns this grid waits for
-  const uint32_t tmem = s_tmem;   // S/P slots at columns 0 and 128, O of tile t at 256 + 128 t
+  const uint32_t tmem = s_tmem;   // S/P of tile t, block j at columns 128 t + 64 (j & 1), O of tile t at 256 + 128 t
   const bool fix_lo = nblk > 0 && blk0 * kFmBlk < vis_lo, fix_hi = nblk > 0 && (blk0 + nblk) * kFmBlk - 1 > vis_hi;
 
   if (warp == 0) {
-    if (items > 0 && elect_one()) {
+    if (nblk > 0 && elect_one()) {
       mbar_expect_tx(b_q, nt * a.nc * a.g * a.tq * 128);
       for (int t = 0; t < nt; t++)
-        for (int c = 0; c < a.nc; c++) tma_load_3d(smem_u32(sQ + (t * a.nc + c) * kFmSlot), &q_map, b_q, c * 64, hkv * a.g, tok0 + t * a.tq);
+        for (int c = 0; c < a.nc; c++) tma_load_3d(smem_u32(sQ + (t * a.nc + c) * kFmQ), &q_map, b_q, c * 64, hkv * a.g, tok0 + t * a.tq);
       int s = 0, group = 0, tail = 0, room = a.slots;      // groups are released in the order of loading
-      auto size_of = [&](int g) { return (nt == 2 ? (g & 1) : g == 2 * nblk - 1 || (g > 0 && !(g & 1))) ? a.nv : a.nc; };
+      auto size_of = [&](int g) { return g == 2 * nblk - 1 || (g > 0 && !(g & 1)) ? a.nv : a.nc; };      // K K V K V .. K V V
       const int* bt = a.block_tables + (long long)seq * a.bt_stride;
       auto load = [&](int j, bool v) -> bool {
         const int key0 = (blk0 + j) * kFmBlk;
-        int pg[2] = {0, 0};
-        if (a.paged)
-#pragma unroll
-          for (int h = 0; h < 2; h++) {      // pages without a visible key (their table entry may be anything) read one that has
-            pg[h] = bt[min(max(key0 / 64 + h, vis_lo / 64), vis_hi / 64)];
-            if (!NE_INDEX_OK(pg[h], BK_CACHE_PAGES, kKernelFm, __LINE__)) pg[h] = 0;
-          }
+        int page = 0;
+        if (a.paged) {
+          page = bt[blk0 + j];
+          if (!NE_INDEX_OK(page, BK_CACHE_PAGES, kKernelFm, __LINE__)) page = 0;
+        }
         const int n = v ? a.nv : a.nc;
         for (; room < n; tail++) {
           if (!mbar_wait(b_empty + 8 * (tail % kFmGroups), (tail / kFmGroups) & 1, abort_flag, kKernelFm, 100)) return false;
@@ -146,8 +152,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
         for (int c = 0; c < n; c++) {
           const uint32_t dst = smem_u32(sKV + s * kFmSlot);
           if (a.paged) {
-            tma_load_4d(dst, v ? &v_map : &k_map, bar, c * 64, hkv, 0, pg[0]);
-            tma_load_4d(dst + kFmSlot / 2, v ? &v_map : &k_map, bar, c * 64, hkv, 0, pg[1]);
+            tma_load_4d(dst, v ? &v_map : &k_map, bar, c * 64, hkv, 0, page);
           } else if (!v && c >= a.rope_chunk) {
             tma_load_2d(dst, &r_map, bar, (c - a.rope_chunk) * 64, k_beg + key0);
           } else {
@@ -160,38 +165,36 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
         return true;
       };
       bool ok = load(0, false);
-      if (ok && nt == 1 && nblk > 1) ok = load(1, false);
-      for (int j = 0; ok && j < nblk; j++) {
-        const int next = j + (nt == 2 ? 1 : 2);
-        ok = load(j, true) && (next >= nblk || load(next, false));
-      }
+      if (ok && nblk > 1) ok = load(1, false);
+      for (int j = 0; ok && j < nblk; j++) ok = load(j, true) && (j + 2 >= nblk || load(j + 2, false));
     }
   } else if (warp <= 2) {
     const int t = warp - 1;       // the issuer's tile
-    if (t < nt && items > 0 && elect_one()) {
+    if (t < nt && nblk > 0 && elect_one()) {
       constexpr uint32_t kIdS = make_idesc(FMT_BF16, FMT_BF16, 128, kFmBlk);
       const uint32_t id_pv = make_idesc(FMT_BF16, FMT_BF16, 128, (uint32_t)a.npv, 0, 1);      // B (= V) is MN-major
       // descriptors of the operands' first tiles; others by adding their distance (in units of 16 bytes)
       constexpr uint32_t kTile = kFmSlot >> 4;
-      const uint64_t dq = make_smem_desc(smem_u32(sQ), 16, 1024, SW_128B) + t * a.nc * kTile, dk = make_smem_desc(smem_u32(sKV), 16, 1024, SW_128B),
+      const uint64_t dq = make_smem_desc(smem_u32(sQ), 16, 1024, SW_128B) + t * a.nc * (kFmQ >> 4), dk = make_smem_desc(smem_u32(sKV), 16, 1024, SW_128B),
                      dv = make_smem_desc(smem_u32(sKV), kFmSlot, 1024, SW_128B);
-      const uint32_t o = tmem + 256 + t * 128;
-      // first slots of the groups in the order of loading (no division: its reciprocal would wait behind the softmax's exponentials)
+      const uint32_t o = tmem + 256 + t * 128, s0 = tmem + t * 128;
+      // groups in the order of loading: number and first slot of the next one (no division: its reciprocal would wait behind the softmax's exponentials)
       int s = 0, group = 0;
-      auto take = [&](int n, int where, int& first, int& bar) -> bool {
-        if (!mbar_wait(b_full + 8 * (group % kFmGroups), (group / kFmGroups) & 1, abort_flag, kKernelFm, where)) return false;
-        first = s; bar = group++ % kFmGroups;
+      auto full = [&](int g) { return b_full + 8 * (g % kFmGroups); };
+      auto parity = [](int g) { return (uint32_t)(g / kFmGroups) & 1; };
+      auto step = [&](int n, int& first, uint32_t& done) {
+        first = s; done = b_empty + 8 * (group++ % kFmGroups);
         s += n;
         if (s >= a.slots) s -= a.slots;
-        return true;
       };
-      int k0 = 0, kb = 0, v0 = 0, vb = 0;
-      auto scores = [&](int n) {
+      int k0 = 0, v0 = 0;
+      uint32_t kd = 0, vd = 0;
+      auto scores = [&](int j) {
         tc_fence_after();
-        const uint32_t d = tmem + (n & 1) * kFmBlk;
+        const uint32_t d = s0 + (j & 1) * kFmBlk;
         int ks = k0;
         for (int c = 0; c < a.nc; c++) {
-          const uint64_t qa = dq + c * kTile, ka = dk + ks * kTile;
+          const uint64_t qa = dq + c * (kFmQ >> 4), ka = dk + ks * kTile;
           const int steps = a.ksteps - 4 * c;
           umma_f16(d, qa, ka, kIdS, c != 0);
           if (steps > 1) umma_f16(d, qa + 2, ka + 2, kIdS, 1);
@@ -199,24 +202,31 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
           if (steps > 3) umma_f16(d, qa + 6, ka + 6, kIdS, 1);
           if (++ks == a.slots) ks = 0;
         }
-        tc_commit(b_s + 8 * (n & 1));
-        tc_commit(b_empty + 8 * kb);
+        tc_commit(b_s + 16 * t + 8 * (j & 1));
+        tc_commit(kd);
       };
-      bool ok = mbar_wait(b_q, 0, abort_flag, kKernelFm, 200) && take(a.nc, 210, k0, kb);
-      if (ok) scores(t);
-      if (ok && nt == 1 && nblk > 1) {
-        ok = take(a.nc, 211, k0, kb);
-        if (ok) scores(1);
+      bool ok = mbar_wait(b_q, 0, abort_flag, kKernelFm, 200);
+      for (int j = 0; ok && j < 2 && j < nblk; j++) {
+        ok = mbar_wait(full(group), parity(group), abort_flag, kKernelFm, 210);
+        step(a.nc, k0, kd);
+        if (ok) scores(j);
       }
       for (int j = 0; ok && j < nblk; j++) {
-        const int n = j * nt + t, next = nt == 2 ? j + 1 : j + 2;      // item n + 2 is block `next` of this tile
-        // the next products' operands are waited for while the softmax works
-        ok = take(a.nv, 220, v0, vb) && (next >= nblk || take(a.nc, 212, k0, kb));
+        const bool next = j + 2 < nblk;
+        const uint32_t bp = b_p + 16 * t + 8 * (j & 1), pp = (j >> 1) & 1;
+        const uint32_t bv = full(group), pv = parity(group), bk = next ? full(group + 1) : bv, pk = next ? parity(group + 1) : pv;
+        bool rv, rk, rp;
+        mbar_test3(bv, pv, bk, pk, bp, pp, rv, rk, rp);      // three tests for the price of one
+        if (!rv) ok = mbar_wait(bv, pv, abort_flag, kKernelFm, 220);
+        if (ok && !rk) ok = mbar_wait(bk, pk, abort_flag, kKernelFm, 212);
         if (ok && j == 0 && fix_lo) ok = mbar_wait(b_fix, 0, abort_flag, kKernelFm, 221);
         if (ok && j == nblk - 1 && fix_hi) ok = mbar_wait(b_fix + 8, 0, abort_flag, kKernelFm, 222);
-        if (!ok || !mbar_wait(b_p + 8 * (n & 1), (n >> 1) & 1, abort_flag, kKernelFm, 230)) break;
+        if (ok && !rp) ok = mbar_wait(bp, pp, abort_flag, kKernelFm, 230);
+        if (!ok) break;
+        step(a.nv, v0, vd);
+        if (next) step(a.nc, k0, kd);
         tc_fence_after();
-        const uint32_t p = tmem + (n & 1) * kFmBlk;
+        const uint32_t p = s0 + (j & 1) * kFmBlk;
         // the chunks of V lie in consecutive ring slots; where they wrap around the ring's end, the product is issued in two column ranges
         const int head = min(a.nv, a.slots - v0);
         const uint64_t va = dv + v0 * kTile;
@@ -224,20 +234,20 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
 #pragma unroll
           for (int x = 0; x < (kSplitP ? 2 : 1); x++)
 #pragma unroll
-            for (int ks = 0; ks < 8; ks++) umma_f16_ts(o, p + x * 64 + ks * 8, va + ks * 128, id_pv, (x | ks) ? 1u : (uint32_t)(j != 0));
+            for (int ks = 0; ks < 4; ks++) umma_f16_ts(o, p + x * 32 + ks * 8, va + ks * 128, id_pv, (x | ks) ? 1u : (uint32_t)(j != 0));
         } else {
           const uint32_t id_a = make_idesc(FMT_BF16, FMT_BF16, 128, (uint32_t)head * 64, 0, 1), id_b = make_idesc(FMT_BF16, FMT_BF16, 128, (uint32_t)(a.npv - head * 64), 0, 1);
 #pragma unroll
           for (int x = 0; x < (kSplitP ? 2 : 1); x++)
 #pragma unroll
-            for (int ks = 0; ks < 8; ks++) {
-              umma_f16_ts(o, p + x * 64 + ks * 8, va + ks * 128, id_a, (x | ks) ? 1u : (uint32_t)(j != 0));
-              umma_f16_ts(o + head * 64, p + x * 64 + ks * 8, dv + ks * 128, id_b, (x | ks) ? 1u : (uint32_t)(j != 0));
+            for (int ks = 0; ks < 4; ks++) {
+              umma_f16_ts(o, p + x * 32 + ks * 8, va + ks * 128, id_a, (x | ks) ? 1u : (uint32_t)(j != 0));
+              umma_f16_ts(o + head * 64, p + x * 32 + ks * 8, dv + ks * 128, id_b, (x | ks) ? 1u : (uint32_t)(j != 0));
             }
         }
-        tc_commit(b_pv + 8 * (n & 1));
-        tc_commit(b_empty + 8 * vb);
-        if (next < nblk) scores(n + 2);
+        tc_commit(b_pv + 16 * t + 8 * (j & 1));
+        tc_commit(vd);
+        if (next) scores(j + 2);
       }
     }
   } else if (warp < 4) {
@@ -245,13 +255,13 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
       if (!(w ? fix_hi : fix_lo)) continue;
       const int j = w ? nblk - 1 : 0, key0 = (blk0 + j) * kFmBlk;
       // group and first slot of the block's V in the order of loading
-      const int g = nt == 2 ? 2 * j + 1 : min(j + 2, nblk) + j, p0 = nt == 2 ? j * (a.nc + a.nv) + a.nc : min(j + 2, nblk) * a.nc + j * a.nv;
+      const int g = min(j + 2, nblk) + j, p0 = min(j + 2, nblk) * a.nc + j * a.nv;
       // once its loads are under way the phase waited for is the current one
       if (mbar_wait(b_go + 8 * w, 0, abort_flag, kKernelFm, 400) && mbar_wait(b_full + 8 * (g % kFmGroups), (g / kFmGroups) & 1, abort_flag, kKernelFm, 410))
         for (int i = (int)lane_id(); i < a.nv * kFmBlk; i += 32) {
           const int key = key0 + (i & (kFmBlk - 1));
           if (w ? key > vis_hi : key < vis_lo) {
-            uint4* dst = reinterpret_cast<uint4*>(sKV + ((p0 + (i >> 7)) % a.slots) * kFmSlot + (i & (kFmBlk - 1)) * 128);
+            uint4* dst = reinterpret_cast<uint4*>(sKV + ((p0 + i / kFmBlk) % a.slots) * kFmSlot + (i & (kFmBlk - 1)) * 128);
 #pragma unroll
             for (int x = 0; x < 8; x++) dst[x] = make_uint4(0, 0, 0, 0);
           }
@@ -270,35 +280,35 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     int last = -1;
-    for (int n = t; ok && t < nt && n < items; n += nt) {
-      const int key0 = (blk0 + (nt == 2 ? n >> 1 : n)) * kFmBlk;
-      const uint32_t ts = tmem + (n & 1) * kFmBlk + lane_addr;
-      if (!mbar_wait(b_s + 8 * (n & 1), (n >> 1) & 1, abort_flag, kKernelFm, 300)) { ok = false; break; }
+    const int own = t < nt ? nblk : 0;
+    const uint32_t bs = b_s + 16 * t, bp = b_p + 16 * t, bpv = b_pv + 16 * t;
+    bool ready = false;
+    for (int j = 0; ok && j < own; j++) {
+      const int key0 = (blk0 + j) * kFmBlk;
+      const uint32_t ts = tmem + t * 128 + (j & 1) * kFmBlk + lane_addr;
+      if (!ready && !mbar_wait(bs + 8 * (j & 1), (j >> 1) & 1, abort_flag, kKernelFm, 300)) { ok = false; break; }
       tc_fence_after();
       __syncwarp();
-      uint32_t r[128];
-#pragma unroll
-      for (int c = 0; c < 4; c++) tmem_ld_32x32b_x32(ts + c * 32, *reinterpret_cast<uint32_t(*)[32]>(r + c * 32));
+      uint32_t r[64];
+      tmem_ld_32x32b_x32(ts, *reinterpret_cast<uint32_t(*)[32]>(r));
+      tmem_ld_32x32b_x32(ts + 32, *reinterpret_cast<uint32_t(*)[32]>(r + 32));
       tc_wait_ld();
       if (key0 + kFmBlk - 1 > limit || key0 < lowest) {
 #pragma unroll
-        for (int j = 0; j < 128; j++)
-          if (key0 + j > limit || key0 + j < lowest) r[j] = 0xff800000u;
+        for (int i = 0; i < 64; i++)
+          if (key0 + i > limit || key0 + i < lowest) r[i] = 0xff800000u;
       }
 #ifdef NE_DEBUG_BOUNDS
-      if (a.paged)                             // the keys of a page that is none take no part
+      if (a.paged && !NE_INDEX_OK(a.block_tables[(long long)seq * a.bt_stride + blk0 + j], BK_CACHE_PAGES, kKernelFm, __LINE__)) {      // keys of a page that is none
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int pg = key0 / 64 + h;
-          if (pg <= vis_hi / 64 && !NE_INDEX_OK(a.block_tables[(long long)seq * a.bt_stride + max(pg, vis_lo / 64)], BK_CACHE_PAGES, kKernelFm, __LINE__)) {
-#pragma unroll
-            for (int j = 0; j < 64; j++) r[h * 64 + j] = 0xff800000u;
-          }
-        }
+        for (int i = 0; i < 64; i++) r[i] = 0xff800000u;
+      }
 #endif
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int j = 0; j < 128; j++) mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(r[j]));
+      for (int i = 0; i < 64; i += 8)
+#pragma unroll
+        for (int e = 0; e < 4; e++) mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(r[i + 2 * e]), __uint_as_float(r[i + 2 * e + 1])));
       float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * a.scale_log2;
       // 32-bit probabilities: the reference is a whole power of two, so rescaling by it is exact and the two terms of a probability are the same whatever the
       // slices and blocks are.  bf16 probabilities: the largest one is exactly 1, and a row that looks at few keys has the smaller error.
@@ -310,10 +320,6 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
       const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
       float ps[2] = {0.f, 0.f};
       __syncwarp();                          // rows at a limit took a branch of their own
-      // the two tiles take turns at the exponentials (warps of one scheduler in pairs): left alone they fall into step, and then neither tile's
-      // products run beside the other's softmax
-      const int turn = n >> 1;
-      if (nt == 2 && (t || turn) && !mbar_wait(b_turn + 8 * (t * 4 + wq), (t ? turn : turn - 1) & 1, abort_flag, kKernelFm, 330)) { ok = false; break; }
       // 32 columns at a time; the next ones' exponentials are under way while these are packed and stored
       auto exps = [&](int c) {
 #pragma unroll
@@ -323,8 +329,8 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
       };
       exps(0);
 #pragma unroll
-      for (int c = 0; c < 4; c++) {
-        if (c < 3) exps(c + 1);
+      for (int c = 0; c < 2; c++) {
+        if (c < 1) exps(c + 1);
         uint32_t* x = r + c * 32;
         uint32_t hi[16];
         if constexpr (kSplitP) {
@@ -335,7 +341,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
             add2(ps, x[2 * j], x[2 * j + 1]);
             lo[j] = pack_bf16x2(__uint_as_float(x[2 * j]) - __uint_as_float(x[2 * j] & 0xffff0000u), __uint_as_float(x[2 * j + 1]) - __uint_as_float(x[2 * j + 1] & 0xffff0000u));
           }
-          tmem_st_32x32b_x16(ts + 64 + c * 16, lo);
+          tmem_st_32x32b_x16(ts + 32 + c * 16, lo);
         } else {
 #pragma unroll
           for (int j = 0; j < 16; j++) {       // sum what the product will see, so numerator and denominator stay consistent
@@ -346,11 +352,11 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
         tmem_st_32x32b_x16(ts + c * 16, hi);
       }
       __syncwarp();
-      if (nt == 2 && lane_id() == 0) mbar_arrive(b_turn + 8 * ((t ^ 1) * 4 + wq));
+      ready = j + 1 < own && mbar_test(bs + 8 * ((j + 1) & 1), ((j + 1) >> 1) & 1);
       l_run = l_run * alpha + (ps[0] + ps[1]);
       m_run = m_new;
       if (last >= 0 && __any_sync(0xffffffffu, alpha < 1.f)) {
-        if (!mbar_wait(b_pv + 8 * (last & 1), (last >> 1) & 1, abort_flag, kKernelFm, 310)) { ok = false; break; }
+        if (!mbar_wait(bpv + 8 * (last & 1), (last >> 1) & 1, abort_flag, kKernelFm, 310)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int cblk = 0; cblk < (a.npv + 15) / 16; cblk++) {
@@ -365,10 +371,10 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane_id() == 0) mbar_arrive(b_p + 8 * (n & 1));
-      last = n;
+      if (lane_id() == 0) mbar_arrive(bp + 8 * (j & 1));
+      last = j;
     }
-    if (ok && last >= 0) ok = mbar_wait(b_pv + 8 * (last & 1), (last >> 1) & 1, abort_flag, kKernelFm, 320);
+    if (ok && last >= 0) ok = mbar_wait(bpv + 8 * (last & 1), (last >> 1) & 1, abort_flag, kKernelFm, 320);
     const bool have = ok && last >= 0;
     const long long rows = (long long)a.T * a.Hq, orow = row_ok ? (long long)(tok0 + tl) * a.Hq + head : 0;
     if (have) tc_fence_after();
@@ -423,7 +429,7 @@ static int fmha_launch(const CUtensorMap& q, const CUtensorMap& k, const CUtenso
     configured = true;
   }
   return (int)launch_pdl(fmha_kernel<kWG, kSplitP>, dim3((unsigned)grid_x, (unsigned)heads, (unsigned)a.splits), dim3(128 + 128 * kWG),
-                         (size_t)(kWG * a.nc + a.slots) * kFmSlot + 1024, st, q, k, v, r, a);
+                         (size_t)kWG * a.nc * kFmQ + (size_t)a.slots * kFmSlot + 1024, st, q, k, v, r, a);
 }
 
 }  // namespace ne
@@ -446,7 +452,7 @@ extern "C" int ne_fmha(const void* q, long long q_ld, const void* k, long long k
   a.g = Hq / Hkv; a.tq = 128 / a.g; a.tiles = tiles; a.splits = splits; a.T = T; a.Hq = Hq;
   a.nc = (D + 63) / 64; a.nv = (Dv + 63) / 64; a.ksteps = (D + 15) / 16; a.npv = (Dv + 15) / 16 * 16; a.dv = Dv;
   a.rope_chunk = k_rope ? k_dim / 64 : a.nc;
-  a.slots = (kFmSmem - 1024) / kFmSlot - tiles * a.nc;
+  a.slots = (kFmSmem - 1024 - tiles * a.nc * kFmQ) / kFmSlot;
   if (a.slots > kFmMaxSlots) a.slots = kFmMaxSlots;
   if (a.slots < a.nc + a.nv) return 1004;                           // a block's K waits for its V, and the next block's K beside it
   a.window = window > 0 ? window : 0; a.causal = causal; a.paged = block_tables != nullptr;
