@@ -1,5 +1,5 @@
 // Grouped-query paged attention on tcgen05 tensor cores: bf16 queries, bf16 paged K / V caches, head dim 128, 64-token
-// pages.  Serves decode steps (one new token per sequence); longer portions run in fmha.cu.
+// pages.  Serves decode steps, verification and short prompts; portions whose tiles fill the SMs run in fmha.cu.
 //
 // One CTA = one KV head x one tile of 128 query rows of ONE sequence x one slice of its key pages.  A row is a
 // (token, query head of the group) pair, r = token_in_tile * g + head_in_group with g = Hq / Hkv (a power of two up to

@@ -235,11 +235,13 @@ def gqa_attention_paged(q, k_cache, v_cache, block_tables, cu_seqlens_q, context
                and k_cache.is_contiguous() and v_cache.is_contiguous())
     if D == 128 and window <= 0 and pages64 and group & (group - 1) == 0:
         q = q.contiguous()
-        if T > B:                                      # some sequence has more than one new token
+        # The prompt kernel where its tiles fill the SMs and the portions fill tiles; else the kernel of the decode steps, whose results are the same.  us for that /
+        # this, 64 / 4 heads: 4 prompts of 1000: 183 / 138, one of 600 (304 tiles): 26 / 20; 8 / 1 heads, one of 2000 (126 tiles): 31 / 38; 128 x 2 tokens: 150 / 172
+        tq = 128 // group
+        if T >= B * tq and min(T, T // tq + B) * Hkv > _sms():
             return _fmha(q, k_cache, v_cache, cu, scale, True, False, bt, cl)
         out = torch.empty(T, Hq, D, dtype=torch.bfloat16, device=q.device)
         # tcgen05 kernel: one CTA per (kv head, tile of 128 (token, head) rows, key slice)
-        tq = 128 // group
         max_tiles = min(T, T // tq + B)
         S = 1
         if max_tiles * Hkv < 74:                       # few CTAs (small decode batches): slice the keys
