@@ -49,6 +49,7 @@ struct FmArgs {
   int nc, nv, ksteps, npv, dv;                 // 64-column chunks of K and V, K = 16 steps of the first product, N of the second, value columns
   int rope_chunk;                              // chunks of K from this one on come from the rotary map, shared by the heads
   int slots, window, causal, paged;
+  uint32_t tmem_cols;
   float scale_log2;
   __nv_bfloat16* out;                          // [T, Hq, dv]
   float* part; float* lse2;                    // [splits, T, Hq, dv], [splits, T, Hq] (splits > 1)
@@ -77,7 +78,7 @@ __device__ __forceinline__ void mbar_test3(uint32_t a, uint32_t pa, uint32_t b, 
 
 // kWG: softmax warpgroups = most tiles per CTA
 template <int kWG, bool kSplitP>
-__global__ void __launch_bounds__(128 + 128 * kWG, 1)
+__global__ void __launch_bounds__(128 + 128 * kWG, kWG == 1 ? 2 : 1)
 fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
             const __grid_constant__ CUtensorMap r_map, const FmArgs a) {
   pdl_wait();                     // dependent launch: nothing above this line touches global memory
@@ -101,7 +102,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
     find_seq_tile(a.cu_seqlens_q, a.num_seqs, a.tq * a.tiles, (int)(gridDim.x - 1 - blockIdx.x), seq, tok);
     if (lane_id() == 0) { s_seq = seq; s_tok = tok; }
   }
-  if (warp == 2) { tmem_alloc(smem_u32(&s_tmem), 512); tmem_relinquish(); }
+  if (warp == 2) { tmem_alloc(smem_u32(&s_tmem), a.tmem_cols); tmem_relinquish(); }
   __syncthreads();
   const int seq = s_seq, tok0 = s_tok;
 
@@ -132,7 +133,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   pdl_trigger();                  // behind the TMEM allocation: a CTA of the next grid never holds columns this grid waits for
-  const uint32_t tmem = s_tmem;   // S/P of tile t, block j at columns 128 t + 64 (j & 1), O of tile t at 256 + 128 t
+  const uint32_t tmem = s_tmem;   // S/P of tile t, block j at columns 128 t + 64 (j & 1), O of tile t behind them at 128 kWG + 128 t
   const bool fix_lo = nblk > 0 && blk0 * kFmBlk < vis_lo, fix_hi = nblk > 0 && (blk0 + nblk) * kFmBlk - 1 > vis_hi;
 
   if (warp == 0) {
@@ -186,7 +187,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
       constexpr uint32_t kTile = kFmSlot >> 4;
       const uint64_t dq = make_smem_desc(smem_u32(sQ), 16, 1024, SW_128B) + t * a.nc * (kFmQ >> 4), dk = make_smem_desc(smem_u32(sKV), 16, 1024, SW_128B),
                      dv = make_smem_desc(smem_u32(sKV), kFmSlot, 1024, SW_128B);
-      const uint32_t o = tmem + 256 + t * 128, s0 = tmem + t * 128;
+      const uint32_t o = tmem + kWG * 128 + t * 128, s0 = tmem + t * 128;
       // groups in the order of loading: number and first slot of the next one (no division: its reciprocal would wait behind the softmax's exponentials)
       int s = 0, group = 0;
       auto full = [&](int g) { return b_full + 8 * (g % kFmGroups); };
@@ -285,7 +286,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
     const bool row_ok = row < a.g * a.tq && tl < n_tok;
     const int limit = row_ok ? (a.causal ? base_limit + tl : base_limit) : -1;
     const int lowest = a.window > 0 ? limit - a.window + 1 : 0;
-    const uint32_t tmem_o = tmem + 256 + t * 128 + lane_addr;
+    const uint32_t tmem_o = tmem + kWG * 128 + t * 128 + lane_addr;
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     int last = -1;
@@ -424,10 +425,11 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
   __syncthreads();
   if (*abort_flag && threadIdx.x == 0) for (int i = 0; i < 2000; i++) __nanosleep(1000);      // copies in flight
   __syncthreads();
-  if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, 512); }
+  if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, a.tmem_cols); }
 }
 
 constexpr int kFmSmem = 232448 - 1024;         // dynamic shared memory limit of a block less the static part
+constexpr int kFmSmemHalf = 233472 / 2 - 2 * 1024;      // where two blocks share an SM (1 KB of each is the system's)
 
 template <int kWG, bool kSplitP>
 static int fmha_launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const CUtensorMap& r, const FmArgs& a, int grid_x, int heads, cudaStream_t st) {
@@ -461,7 +463,10 @@ extern "C" int ne_fmha(const void* q, long long q_ld, const void* k, long long k
   a.g = Hq / Hkv; a.tq = 128 / a.g; a.tiles = tiles; a.splits = splits; a.T = T; a.Hq = Hq;
   a.nc = (D + 63) / 64; a.nv = (Dv + 63) / 64; a.ksteps = (D + 15) / 16; a.npv = (Dv + 15) / 16 * 16; a.dv = Dv;
   a.rope_chunk = k_rope ? k_dim / 64 : a.nc;
-  a.slots = (kFmSmem - 1024 - tiles * a.nc * kFmQ) / kFmSlot;
+  // single tiles: two CTAs share an SM where TMEM has room for both (one's loads and epilogue run beside the other's work)
+  const bool share = tiles == 1 && Dv <= 128 && D <= 192;
+  a.tmem_cols = share ? 256 : 512;
+  a.slots = ((share ? kFmSmemHalf : kFmSmem) - 1024 - tiles * a.nc * kFmQ) / kFmSlot;
   if (a.slots > kFmMaxSlots) a.slots = kFmMaxSlots;
   if (a.slots < a.nc + a.nv) return 1004;                           // a block's K waits for its V, and the next block's K beside it
   a.window = window > 0 ? window : 0; a.causal = causal; a.paged = block_tables != nullptr;

@@ -181,16 +181,16 @@ def _fmha_covers(group: int, D: int, Dv: int) -> bool:
     return 1 <= group <= 128 and 8 <= D <= 256 and D % 8 == 0 and 8 <= Dv <= 256 and Dv % 8 == 0
 
 
-def _fmha(q, k, v, cu, scale, causal, split_p, block_tables=None, context_lens=None, window=0, k_rope=None, one_token=False):
+def _fmha(q, k, v, cu, scale, causal, split_p, block_tables=None, context_lens=None, window=0, k_rope=None):
     """The tcgen05 prompt kernel, for sizes that `_fmha_covers`; rows and pages as the kernel's entry wants them."""
     T, Hq, D = q.shape
     paged = block_tables is not None
     Hkv, Dv = (k.shape[2], v.shape[3]) if paged else (k.shape[1], v.shape[2])
     B = cu.numel() - 1
     tq = 128 // (Hq // Hkv)
-    # two tiles per CTA: one's softmax runs beside the other's products; TMEM holds two accumulators of up to 128 columns, shared memory two Q tiles of up to
-    # 192.  One tile where pairs would leave SMs idle (and where a sequence has only one).
-    tiles = 1 if one_token or Dv > 128 or D > 192 or min(T, T // (2 * tq) + B) * Hkv < _sms() else 2
+    # Two tiles per CTA share the keys they read; TMEM holds two accumulators of up to 128 columns, shared memory two Q tiles of up to 192.  One tile where
+    # single ones fit a wave or a portion is less than one; us for one / two (MLA): a prompt of 2000, 16 heads: 68 / 48; 8 of 64, 128 heads: 40 / 57
+    tiles = 1 if Dv > 128 or D > 192 or T < B * tq or min(T, T // tq + B) * Hkv <= _sms() else 2
     rows = tq * tiles
     grid = min(T, T // rows + B)
     S = 1
@@ -260,7 +260,7 @@ def gqa_attention_paged(q, k_cache, v_cache, block_tables, cu_seqlens_q, context
     assert group % 4 == 0 or group == 1 and Hq % 4 == 0 or Hkv == Hq, "query heads per kv head must be a multiple of 4"
     if (pages64 and scale > 0 and _fmha_covers(group, D, D) and k_cache.shape[3] == v_cache.shape[3] == D and k_cache.data_ptr() % 16 == 0
             and v_cache.data_ptr() % 16 == 0):
-        return _fmha(q if _rows16(q) else q.clone(memory_format=torch.contiguous_format), k_cache, v_cache, cu, scale, True, True, bt, cl, window, one_token=T <= B)
+        return _fmha(q if _rows16(q) else q.clone(memory_format=torch.contiguous_format), k_cache, v_cache, cu, scale, True, True, bt, cl, window)
     out = torch.empty(T, Hq, D, dtype=torch.bfloat16, device=q.device)
     _k._ck(lib.ne_attn_generic(_k._p(q), _c.c_longlong(q.stride(0)), _c.c_int(q.stride(1)), _k._p(k_cache), _k._p(v_cache),
                                _c.c_longlong(Hkv * D), _c.c_int(D), _c.c_int(group), _k._p(bt), _c.c_int(bt.stride(0)), _c.c_int(k_cache.shape[1]),
