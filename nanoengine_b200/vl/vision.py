@@ -9,7 +9,7 @@ Parity: reference vl/vision/encoder.py - rotary table :41-72, MLP :75-91, patch 
 :154-198, block :201-230, model :233-465 (rot_pos_emb :308-352, position interpolation :354-423, forward :425-465).
 
 B200-first differences: every product goes through the tcgen05 GEMM of this package, LayerNorm / GELU / rotary are its CUDA
-kernels, and attention addresses q / k / v in place through the generic paged-attention kernel (one row per "page", no padding
+kernels, and attention addresses q / k / v in place through the ragged tensor-core kernel (no padding
 to the longest image, no per-image Python loop).
 """
 from __future__ import annotations
