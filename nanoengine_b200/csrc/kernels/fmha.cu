@@ -3,15 +3,17 @@
 // last keys; keys and values in 64-token cache pages, or as rows of the same ragged tokens (vision encoders, prompts without a cached prefix).
 //
 // One CTA = one KV head x up to two tiles of 128 (token, head of the group) rows of ONE sequence x one slice of its keys, in blocks of 64 keys (a page).
-// Every tile t has two TMEM score slots of 64 columns, block j in slot j & 1, and a thread that issues its products in the order S(0) S(1), then
-// PV(j) S(j+2) ..:
+// Every tile t has two TMEM score slots of 64 columns (three where one tile has all of TMEM), block j in slot j mod their number, and a thread that issues its
+// products in the order S(0) S(1), then PV(j) S(j+2) ..:
 //     S(j) = Q K^T        (tcgen05.mma kind::f16, M = 128, N = 64, K = 16 steps up to the head size, so a head of 72 pays for 80)
 //     P(j) = exp2(S - m)  one warpgroup per tile; bf16 pairs written over S(j) in TMEM, the A operand of the second product
 //     O   += P(j) V       (N = head size up to the next multiple of 16; V read MN-major)
-// They complete in order, so S(j+2) may overwrite P(j) without a barrier, and the softmax finds S(j+1) ready when it has handed P(j) on.  (Blocks of 128
-// keys with one slot a tile read less shared memory per product, but then scores, softmax and products of a tile are one chain: 4150 cycles for 128 keys of
-// two tiles, whether one or two warpgroups share a tile's softmax; so it is 3900.  One tile per CTA and two CTAs per SM, or an issuer each for scores and
-// products, were no faster.)
+// The softmax finds S(j+1) ready when it has handed P(j) on.  (Blocks of 128 keys with one slot a tile read less shared memory per product, but then scores,
+// softmax and products of a tile are one chain: 4150 cycles for 128 keys of two tiles, whether one or two warpgroups share a tile's softmax; so it is 4000.  One
+// tile per CTA and two CTAs per SM, or an issuer each for scores and products, were no faster.)
+// The order of two products is promised only where they share accumulator and shape, so S(j+2) waits for the products that read the slot: PV(j) itself with two
+// slots, which the other tile's products, or the other CTA's, fill (1063 -> 1088 us for the MLA prompts below, against issuing without the wait), PV(j-1) with
+// three (256-wide heads, nothing beside them: 177 without a wait, 197 with two slots, 186 so).
 // A barrier test costs an issuing thread 300 cycles once products are queued before it, hence an issuer per tile, and tests in threes.
 // kSplitP: probabilities stay 32-bit in effect: bf16 head and bf16 remainder (2^-17), two products against V.  Taken where the plain kernel this one
 // replaced kept them in fp32.
@@ -76,9 +78,9 @@ __device__ __forceinline__ void mbar_test3(uint32_t a, uint32_t pa, uint32_t b, 
   ra = x; rb = y; rc = z;
 }
 
-// kWG: softmax warpgroups = most tiles per CTA
-template <int kWG, bool kSplitP>
-__global__ void __launch_bounds__(128 + 128 * kWG, kWG == 1 ? 2 : 1)
+// kWG: softmax warpgroups = most tiles per CTA; kSlots: score slots of a tile
+template <int kWG, bool kSplitP, int kSlots>
+__global__ void __launch_bounds__(128 + 128 * kWG, kWG == 1 && kSlots == 2 ? 2 : 1)
 fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
             const __grid_constant__ CUtensorMap r_map, const FmArgs a) {
   pdl_wait();                     // dependent launch: nothing above this line touches global memory
@@ -87,13 +89,16 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;                                    // [tile][chunk][128 rows x 128 B]
   uint8_t* sKV = sQ + kWG * a.nc * kFmQ;
-  __shared__ uint64_t bars[2 * kFmGroups + 17];
+  __shared__ uint64_t bars[2 * kFmGroups + 5 + 3 * kWG * kSlots];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort, s_seq, s_tok;
   volatile int* abort_flag = &s_abort;
-  // scores, probabilities, products: [tile][block & 1]
-  const uint32_t b_full = smem_u32(bars), b_empty = b_full + 8 * kFmGroups, b_q = b_empty + 8 * kFmGroups, b_s = b_q + 8, b_p = b_s + 32, b_pv = b_p + 32,
-                 b_go = b_pv + 32, b_fix = b_go + 16;
+  // scores, probabilities, products: [tile][slot]
+  constexpr int kBars = 8 * kWG * kSlots;
+  const uint32_t b_full = smem_u32(bars), b_empty = b_full + 8 * kFmGroups, b_q = b_empty + 8 * kFmGroups, b_s = b_q + 8, b_p = b_s + kBars, b_pv = b_p + kBars,
+                 b_go = b_pv + kBars, b_fix = b_go + 16;
+  auto slot_of = [](int j) { return kSlots == 2 ? j & 1 : j % kSlots; };
+  auto phase_of = [](int j) { return (uint32_t)(j / kSlots) & 1; };
   const int warp = threadIdx.x >> 5;
   const int hkv = blockIdx.y, split = blockIdx.z;
   if (warp == 0) {
@@ -124,7 +129,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
   if (threadIdx.x == 32) {
     for (int i = 0; i < kFmGroups; i++) { mbar_init(b_full + 8 * i, 1); mbar_init(b_empty + 8 * i, nt); }
     mbar_init(b_q, 1);
-    for (int i = 0; i < 4; i++) { mbar_init(b_s + 8 * i, 1); mbar_init(b_p + 8 * i, 4); mbar_init(b_pv + 8 * i, 1); }
+    for (int i = 0; i < kWG * kSlots; i++) { mbar_init(b_s + 8 * i, 1); mbar_init(b_p + 8 * i, 4); mbar_init(b_pv + 8 * i, 1); }
     for (int i = 0; i < 2; i++) { mbar_init(b_go + 8 * i, 1); mbar_init(b_fix + 8 * i, 32); }
     s_abort = 0;
     mbar_fence_init();
@@ -133,7 +138,8 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   pdl_trigger();                  // behind the TMEM allocation: a CTA of the next grid never holds columns this grid waits for
-  const uint32_t tmem = s_tmem;   // S/P of tile t, block j at columns 128 t + 64 (j & 1), O of tile t behind them at 128 kWG + 128 t
+  constexpr uint32_t kO = kSlots == 2 ? 128 * kWG : 256;
+  const uint32_t tmem = s_tmem;   // S/P of tile t, block j at columns 128 t + 64 slot(j), O of tile t behind them at kO + 128 t
   const bool fix_lo = nblk > 0 && blk0 * kFmBlk < vis_lo, fix_hi = nblk > 0 && (blk0 + nblk) * kFmBlk - 1 > vis_hi;
 
   if (warp == 0) {
@@ -187,7 +193,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
       constexpr uint32_t kTile = kFmSlot >> 4;
       const uint64_t dq = make_smem_desc(smem_u32(sQ), 16, 1024, SW_128B) + t * a.nc * (kFmQ >> 4), dk = make_smem_desc(smem_u32(sKV), 16, 1024, SW_128B),
                      dv = make_smem_desc(smem_u32(sKV), kFmSlot, 1024, SW_128B);
-      const uint32_t o = tmem + kWG * 128 + t * 128, s0 = tmem + t * 128;
+      const uint32_t o = tmem + kO + t * 128, s0 = tmem + t * 128, bs = b_s + 8 * kSlots * t, bp = b_p + 8 * kSlots * t, bpv = b_pv + 8 * kSlots * t;
       // groups in the order of loading: number and first slot of the next one (no division: its reciprocal would wait behind the softmax's exponentials)
       int s = 0, group = 0;
       auto full = [&](int g) { return b_full + 8 * (g % kFmGroups); };
@@ -199,9 +205,10 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
       };
       int k0 = 0, v0 = 0;
       uint32_t kd = 0, vd = 0;
+      bool split_before = false;
       auto scores = [&](int j) {
         tc_fence_after();
-        const uint32_t d = s0 + (j & 1) * kFmBlk;
+        const uint32_t d = s0 + slot_of(j) * kFmBlk;
         int ks = k0;
         for (int c = 0; c < a.nc; c++) {
           const uint64_t qa = dq + c * (kFmQ >> 4), ka = dk + ks * kTile;
@@ -212,7 +219,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
           if (steps > 3) umma_f16(d, qa + 6, ka + 6, kIdS, 1);
           if (++ks == a.slots) ks = 0;
         }
-        tc_commit(b_s + 16 * t + 8 * (j & 1));
+        tc_commit(bs + 8 * slot_of(j));
         tc_commit(kd);
       };
       bool ok = mbar_wait(b_q, 0, abort_flag, kKernelFm, 200);
@@ -223,22 +230,25 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
       }
       for (int j = 0; ok && j < nblk; j++) {
         const bool next = j + 2 < nblk;
-        const uint32_t bp = b_p + 16 * t + 8 * (j & 1), pp = (j >> 1) & 1;
+        const uint32_t bj = bp + 8 * slot_of(j), pp = phase_of(j);
         const uint32_t bv = full(group), pv = parity(group), bk = next ? full(group + 1) : bv, pk = next ? parity(group + 1) : pv;
         bool rv, rk, rp;
-        mbar_test3(bv, pv, bk, pk, bp, pp, rv, rk, rp);      // three tests for the price of one
+        mbar_test3(bv, pv, bk, pk, bj, pp, rv, rk, rp);      // three tests for the price of one
         if (!rv) ok = mbar_wait(bv, pv, abort_flag, kKernelFm, 220);
         if (ok && !rk) ok = mbar_wait(bk, pk, abort_flag, kKernelFm, 212);
         if (ok && j == 0 && fix_lo) ok = mbar_wait(b_fix, 0, abort_flag, kKernelFm, 221);
         if (ok && j == nblk - 1 && fix_hi) ok = mbar_wait(b_fix + 8, 0, abort_flag, kKernelFm, 222);
-        if (ok && !rp) ok = mbar_wait(bp, pp, abort_flag, kKernelFm, 230);
-        if (!ok) break;
+        if (ok && !rp) ok = mbar_wait(bj, pp, abort_flag, kKernelFm, 230);
         step(a.nv, v0, vd);
         if (next) step(a.nc, k0, kd);
-        tc_fence_after();
-        const uint32_t p = s0 + (j & 1) * kFmBlk;
-        // the chunks of V lie in consecutive ring slots; where they wrap around the ring's end, the product is issued in two column ranges
         const int head = min(a.nv, a.slots - v0);
+        // products of other column ranges than those of the block before add to the same O: behind them
+        if (ok && kSlots == 3 && j > 0 && (head != a.nv || split_before)) ok = mbar_wait(bpv + 8 * slot_of(j - 1), phase_of(j - 1), abort_flag, kKernelFm, 242);
+        split_before = head != a.nv;
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t p = s0 + slot_of(j) * kFmBlk;
+        // the chunks of V lie in consecutive ring slots; where they wrap around the ring's end, the product is issued in two column ranges
         const uint64_t va = dv + v0 * kTile;
         if (head == a.nv) {
 #pragma unroll
@@ -255,9 +265,11 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
               umma_f16_ts(o + head * 64, p + x * 32 + ks * 8, dv + ks * 128, id_b, (x | ks) ? 1u : (uint32_t)(j != 0));
             }
         }
-        tc_commit(b_pv + 16 * t + 8 * (j & 1));
+        tc_commit(bpv + 8 * slot_of(j));
         tc_commit(vd);
-        if (next) scores(j + 2);
+        // the products whose probabilities lie in the next scores' slot; with two slots these very ones, which also orders them before the next products
+        if (kSlots == 2 ? j + 1 < nblk : next && j > 0) ok = mbar_wait(bpv + 8 * slot_of(j - (kSlots - 2)), phase_of(j - (kSlots - 2)), abort_flag, kKernelFm, 241, 0);
+        if (ok && next) scores(j + 2);
       }
     }
   } else if (warp < 4) {
@@ -286,17 +298,17 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
     const bool row_ok = row < a.g * a.tq && tl < n_tok;
     const int limit = row_ok ? (a.causal ? base_limit + tl : base_limit) : -1;
     const int lowest = a.window > 0 ? limit - a.window + 1 : 0;
-    const uint32_t tmem_o = tmem + kWG * 128 + t * 128 + lane_addr;
+    const uint32_t tmem_o = tmem + kO + t * 128 + lane_addr;
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     int last = -1;
     const int own = t < nt ? nblk : 0;
-    const uint32_t bs = b_s + 16 * t, bp = b_p + 16 * t, bpv = b_pv + 16 * t;
+    const uint32_t bs = b_s + 8 * kSlots * t, bp = b_p + 8 * kSlots * t, bpv = b_pv + 8 * kSlots * t;
     bool ready = false;
     for (int j = 0; ok && j < own; j++) {
       const int key0 = (blk0 + j) * kFmBlk;
-      const uint32_t ts = tmem + t * 128 + (j & 1) * kFmBlk + lane_addr;
-      if (!ready && !mbar_wait(bs + 8 * (j & 1), (j >> 1) & 1, abort_flag, kKernelFm, 300)) { ok = false; break; }
+      const uint32_t ts = tmem + t * 128 + slot_of(j) * kFmBlk + lane_addr;
+      if (!ready && !mbar_wait(bs + 8 * slot_of(j), phase_of(j), abort_flag, kKernelFm, 300)) { ok = false; break; }
       tc_fence_after();
       __syncwarp();
       uint32_t r[64];
@@ -362,11 +374,11 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
         tmem_st_32x32b_x16(ts + c * 16, hi);
       }
       __syncwarp();
-      ready = j + 1 < own && mbar_test(bs + 8 * ((j + 1) & 1), ((j + 1) >> 1) & 1);
+      ready = j + 1 < own && mbar_test(bs + 8 * slot_of(j + 1), phase_of(j + 1));
       l_run = l_run * alpha + (ps[0] + ps[1]);
       m_run = m_new;
       if (last >= 0 && __any_sync(0xffffffffu, alpha < 1.f)) {
-        if (!mbar_wait(bpv + 8 * (last & 1), (last >> 1) & 1, abort_flag, kKernelFm, 310)) { ok = false; break; }
+        if (!mbar_wait(bpv + 8 * slot_of(last), phase_of(last), abort_flag, kKernelFm, 310)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int cblk = 0; cblk < (a.npv + 15) / 16; cblk++) {
@@ -381,10 +393,10 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane_id() == 0) mbar_arrive(bp + 8 * (j & 1));
+      if (lane_id() == 0) mbar_arrive(bp + 8 * slot_of(j));
       last = j;
     }
-    if (ok && last >= 0) ok = mbar_wait(bpv + 8 * (last & 1), (last >> 1) & 1, abort_flag, kKernelFm, 320);
+    if (ok && last >= 0) ok = mbar_wait(bpv + 8 * slot_of(last), phase_of(last), abort_flag, kKernelFm, 320);
     const bool have = ok && last >= 0;
     const long long rows = (long long)a.T * a.Hq, orow = row_ok ? (long long)(tok0 + tl) * a.Hq + head : 0;
     if (have) tc_fence_after();
@@ -431,15 +443,15 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
 constexpr int kFmSmem = 232448 - 1024;         // dynamic shared memory limit of a block less the static part
 constexpr int kFmSmemHalf = 233472 / 2 - 2 * 1024;      // where two blocks share an SM (1 KB of each is the system's)
 
-template <int kWG, bool kSplitP>
+template <int kWG, bool kSplitP, int kSlots>
 static int fmha_launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const CUtensorMap& r, const FmArgs& a, int grid_x, int heads, cudaStream_t st) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(fmha_kernel<kWG, kSplitP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFmSmem);
+    cudaError_t e = cudaFuncSetAttribute(fmha_kernel<kWG, kSplitP, kSlots>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFmSmem);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  return (int)launch_pdl(fmha_kernel<kWG, kSplitP>, dim3((unsigned)grid_x, (unsigned)heads, (unsigned)a.splits), dim3(128 + 128 * kWG),
+  return (int)launch_pdl(fmha_kernel<kWG, kSplitP, kSlots>, dim3((unsigned)grid_x, (unsigned)heads, (unsigned)a.splits), dim3(128 + 128 * kWG),
                          (size_t)kWG * a.nc * kFmQ + (size_t)a.slots * kFmSlot + 1024, st, q, k, v, r, a);
 }
 
@@ -498,6 +510,7 @@ extern "C" int ne_fmha(const void* q, long long q_ld, const void* k, long long k
     uint32_t box[2] = {64, kFmBlk};
     int rc = make_tmap(&mr, k_rope, TMA_BF16, 2, dims, strides, box, TMA_SW_128); if (rc) return 2200 + rc;
   }
-  if (tiles == 2) return split_p ? fmha_launch<2, true>(mq, mk, mv, mr, a, grid_x, Hkv, st) : fmha_launch<2, false>(mq, mk, mv, mr, a, grid_x, Hkv, st);
-  return split_p ? fmha_launch<1, true>(mq, mk, mv, mr, a, grid_x, Hkv, st) : fmha_launch<1, false>(mq, mk, mv, mr, a, grid_x, Hkv, st);
+  if (tiles == 2) return split_p ? fmha_launch<2, true, 2>(mq, mk, mv, mr, a, grid_x, Hkv, st) : fmha_launch<2, false, 2>(mq, mk, mv, mr, a, grid_x, Hkv, st);
+  if (share) return split_p ? fmha_launch<1, true, 2>(mq, mk, mv, mr, a, grid_x, Hkv, st) : fmha_launch<1, false, 2>(mq, mk, mv, mr, a, grid_x, Hkv, st);
+  return split_p ? fmha_launch<1, true, 3>(mq, mk, mv, mr, a, grid_x, Hkv, st) : fmha_launch<1, false, 3>(mq, mk, mv, mr, a, grid_x, Hkv, st);
 }

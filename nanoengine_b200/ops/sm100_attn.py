@@ -181,16 +181,20 @@ def _fmha_covers(group: int, D: int, Dv: int) -> bool:
     return 1 <= group <= 128 and 8 <= D <= 256 and D % 8 == 0 and 8 <= Dv <= 256 and Dv % 8 == 0
 
 
+def _fmha_tiles(T: int, B: int, Hq: int, Hkv: int, D: int, Dv: int) -> int:
+    """Tiles of 128 rows per CTA.  Two share the keys they read; TMEM holds two accumulators of up to 128 columns, shared memory two Q tiles of up to 192.  One
+    where single ones fit a wave or a portion is less than one; us for one / two (MLA): a prompt of 2000, 16 heads: 68 / 48; 8 of 64, 128 heads: 40 / 57"""
+    tq = 128 // (Hq // Hkv)
+    return 1 if Dv > 128 or D > 192 or T < B * tq or min(T, T // tq + B) * Hkv <= _sms() else 2
+
+
 def _fmha(q, k, v, cu, scale, causal, split_p, block_tables=None, context_lens=None, window=0, k_rope=None):
     """The tcgen05 prompt kernel, for sizes that `_fmha_covers`; rows and pages as the kernel's entry wants them."""
     T, Hq, D = q.shape
     paged = block_tables is not None
     Hkv, Dv = (k.shape[2], v.shape[3]) if paged else (k.shape[1], v.shape[2])
     B = cu.numel() - 1
-    tq = 128 // (Hq // Hkv)
-    # Two tiles per CTA share the keys they read; TMEM holds two accumulators of up to 128 columns, shared memory two Q tiles of up to 192.  One tile where
-    # single ones fit a wave or a portion is less than one; us for one / two (MLA): a prompt of 2000, 16 heads: 68 / 48; 8 of 64, 128 heads: 40 / 57
-    tiles = 1 if Dv > 128 or D > 192 or T < B * tq or min(T, T // tq + B) * Hkv <= _sms() else 2
+    tq, tiles = 128 // (Hq // Hkv), _fmha_tiles(T, B, Hq, Hkv, D, Dv)
     rows = tq * tiles
     grid = min(T, T // rows + B)
     S = 1

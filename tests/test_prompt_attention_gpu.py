@@ -85,6 +85,47 @@ def test_ragged(heads, dim, causal, lens):
     assert _rel(got, want) < EXACT_P
 
 
+# more than 32 blocks of 64 keys a CTA, so that every barrier of the ring is used again: (heads, size, lengths, prefix of the first, window, tiles a CTA takes)
+@pytest.mark.parametrize("hq,hkv,dim,new,before,window,tiles", [(32, 8, 128, [1500, 333], 900, 512, 2), (32, 8, 128, [1300, 1000], 0, 2000, 2), (16, 2, 256, [1100, 300], 1500, 0, 1),
+                                                                (16, 4, 256, [900, 500], 2500, 1900, 1), (32, 4, 64, [400, 70], 2700, 0, 1), (32, 4, 64, [2100, 800], 300, 0, 2)])
+def test_long_paged(hq, hkv, dim, new, before, window, tiles):
+    from nanoengine_b200.ops import sm100, sm100_attn
+    sm100.clear_kernel_status()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    total = [new[0] + before, *new[1:]]
+    nb = [-(-n // 64) for n in total]
+    bt = torch.zeros(len(new), max(nb), dtype=torch.int32, device="cuda")
+    kc, vc = (torch.randn(sum(nb), 64, hkv, dim, generator=g, device="cuda").to(torch.bfloat16) for _ in "kv")
+    q = torch.randn(sum(new), hq, dim, generator=g, device="cuda").to(torch.bfloat16) * 3
+    want, at, o = [], 0, 0
+    for i, (n, m) in enumerate(zip(new, total)):
+        bt[i, : nb[i]] = torch.arange(at, at + nb[i], device="cuda")
+        k, v = (x[at: at + nb[i]].reshape(-1, hkv, dim)[:m] for x in (kc, vc))
+        want.append(_attend(q[o: o + n], k, v, dim ** -0.5, m - n, window))
+        at, o = at + nb[i], o + n
+    cu, cl = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([0] + torch.tensor(new).cumsum(0).tolist(), total))
+    assert sm100_attn._fmha_tiles(sum(new), len(new), hq, hkv, dim, dim) == tiles
+    got = sm100_attn.gqa_attention_paged(q, kc, vc, bt, cu, cl, dim ** -0.5, window)
+    assert sm100.kernel_status()[0] == 0 and _rel(got, torch.cat(want)) < EXACT_P
+    assert torch.equal(got, sm100_attn.gqa_attention_paged(q, kc, vc, bt, cu, cl, dim ** -0.5, window))
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("heads,dim,lens,tiles", [(16, 72, [1300, 1201, 77], 2), (8, 72, [2200], 1), (3, 136, [2300, 40], 1), (16, 128, [2500, 130], 2)])
+def test_long_ragged(heads, dim, lens, tiles, causal):
+    from nanoengine_b200.ops import sm100, sm100_attn
+    sm100.clear_kernel_status()
+    g = torch.Generator(device="cuda").manual_seed(6)
+    q, k, v = torch.randn(sum(lens), 3, heads, dim, generator=g, device="cuda").to(torch.bfloat16).unbind(1)
+    at = [0] + torch.tensor(lens).cumsum(0).tolist()
+    cu = torch.tensor(at, dtype=torch.int32, device="cuda")
+    want = torch.cat([_attend(3 * q[a:b], k[a:b], v[a:b], dim ** -0.5, 0, 0, causal) for a, b in zip(at, at[1:])])
+    assert sm100_attn._fmha_tiles(sum(lens), len(lens), heads, heads, dim, dim) == tiles
+    got = sm100.attention_varlen(3 * q, k, v, cu, dim ** -0.5, causal)
+    assert sm100.kernel_status()[0] == 0 and _rel(got, want) < EXACT_P
+    assert torch.equal(got, sm100.attention_varlen(3 * q, k, v, cu, dim ** -0.5, causal))
+
+
 def test_a_sequence_does_not_see_its_neighbour_s_infinities():
     from nanoengine_b200.ops import sm100
     x = torch.randn(3, 200, 4, 72, device="cuda").to(torch.bfloat16)
