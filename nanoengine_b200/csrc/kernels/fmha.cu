@@ -19,8 +19,8 @@
 // replaced kept them in fp32.
 // Shared memory: Q, then a ring of 8 KB slots (64 keys x 64 columns) shared by K and V, loaded in the order of first use; the chunks of a block's K
 // or V (a group) share one barrier.
-// Rows of V in front of the window or past the last visible key (pages that belong to nobody, rows of the next sequence) are zeroed in shared
-// memory before their product: 0 x inf there would reach the result.  Warp 0: TMA producer, 1 and 2: MMA issuers of tile 0 and 1, 3: that zeroing,
+// Rows of V in front of the window or past the last visible key (pages that belong to nobody, rows of the next sequence: often no numbers) are zeroed in shared
+// memory before their product: 0 x inf there would reach the result.  Values that some rows of a tile see and others do not: fmha_row_again.  Warp 0: TMA producer, 1 and 2: MMA issuers of tile 0 and 1, 3: that zeroing,
 // 4-7 / 8-11: softmax, rescale and epilogue of tile 0 / 1.  All waits are bounded.
 //
 // Bound: products issued on their own (no softmax) take 75 - 85 % of the time; 64 keys of two tiles take 1960 cycles, of which the tensor pipe could do with
@@ -55,6 +55,10 @@ struct FmArgs {
   float scale_log2;
   __nv_bfloat16* out;                          // [T, Hq, dv]
   float* part; float* lse2;                    // [splits, T, Hq, dv], [splits, T, Hq] (splits > 1)
+  // the operands again, for rows that are taken once more on the CUDA cores: k rows k_dim wide, then those of the rotary map up to d; heads k_dim / dv apart
+  const __nv_bfloat16* q; const __nv_bfloat16* k; const __nv_bfloat16* v; const __nv_bfloat16* k_rope;
+  long long q_ld, k_ld, v_ld, r_ld;            // k_ld, v_ld: from one token to the next (pages too)
+  int d, k_dim;
 };
 
 // (x, y) <- (x, y) scale + shift, and sum += (x, y): two fp32 operations in one instruction
@@ -78,11 +82,97 @@ __device__ __forceinline__ void mbar_test3(uint32_t a, uint32_t pa, uint32_t b, 
   ra = x; rb = y; rc = z;
 }
 
+// sum of a[i] b[i], n a multiple of 8, both on 16-byte boundaries
+__device__ __forceinline__ float fm_dot(const __nv_bfloat16* a, const __nv_bfloat16* b, int n) {
+  float s = 0.f;
+#pragma unroll 1
+  for (int i = 0; i < n; i += 8) {
+    const uint4 x = *reinterpret_cast<const uint4*>(a + i), y = *reinterpret_cast<const uint4*>(b + i);
+    const uint32_t wx[4] = {x.x, x.y, x.z, x.w}, wy[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const float2 f = unpack_bf16x2(wx[e]), g = unpack_bf16x2(wy[e]);
+      s = fmaf(f.x, g.x, fmaf(f.y, g.y, s));
+    }
+  }
+  return s;
+}
+
+// One row once more, by a warp on the CUDA cores: keys [lo, hi] of the sequence's page table `bt` (or its own tokens, k_beg on).  A tile's products multiply every
+// value row that one of its rows sees; zero times an infinity, or no number, among those that others may not see reaches them, an infinity's two terms may have
+// opposite signs, and a sum may overflow before it is divided.  So a row whose sums are not all finite is taken again, values of probability zero left out.  m, inv:
+// reference exponent and 1 / sum of the row, which come from scores alone and stand (inv 0: no key).  Never reached with finite values, and rolled up, so that it
+// costs the loops of the kernel no register (107 -> 106; as a call, or at the end for all warps, it cost 2 % of the MLA prompts' time, so nothing).
+template <bool kSplitP>
+__device__ __forceinline__ void fmha_row_again(const FmArgs& a, const int* bt, int k_beg, int hkv, long long tok, int head, int lo, int hi, float m, float inv, int split) {
+  const int lane = (int)lane_id();
+  const __nv_bfloat16* q = a.q + tok * a.q_ld + (long long)head * a.d;
+  float acc[8];                              // columns 64 i + 2 lane and the next
+#pragma unroll
+  for (int i = 0; i < 8; i++) acc[i] = 0.f;
+  auto token = [&](int key) -> long long {   // row of the key, -1: of a page that is none
+    if (!a.paged) return k_beg + key;
+    const int page = bt[key / kFmBlk];
+    return NE_INDEX_OK(page, BK_CACHE_PAGES, kKernelFm, __LINE__) ? (long long)page * kFmBlk + key % kFmBlk : -1;
+  };
+#pragma unroll 1
+  for (int key0 = inv > 0.f ? lo : hi + 1; key0 <= hi; key0 += 32) {
+    const long long row = key0 + lane <= hi ? token(key0 + lane) : -1;
+    float w = 0.f;
+    if (row >= 0) {
+      float s = fm_dot(q, a.k + row * a.k_ld + (long long)hkv * a.k_dim, a.k_dim);
+      if (a.k_dim < a.d) s += fm_dot(q + a.k_dim, a.k_rope + row * a.r_ld, a.d - a.k_dim);
+      w = exp2f(fmaf(s, a.scale_log2, -m));
+      if (!kSplitP) w = __bfloat162float(__float2bfloat16(w));
+      w *= inv;
+    }
+#pragma unroll 1
+    for (int e = 0; e < 32; e++) {
+      const float we = __shfl_sync(0xffffffffu, w, e);
+      const long long re = __shfl_sync(0xffffffffu, row, e);
+      if (we == 0.f) continue;
+      const __nv_bfloat16* v = a.v + re * a.v_ld + (long long)hkv * a.dv;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int c = 64 * i + 2 * lane;
+        if (c < a.dv) {
+          const float2 f = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(v + c));
+          acc[2 * i] = fmaf(we, f.x, acc[2 * i]); acc[2 * i + 1] = fmaf(we, f.y, acc[2 * i + 1]);
+        }
+      }
+    }
+  }
+  const long long orow = tok * a.Hq + head;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int c = 64 * i + 2 * lane;
+    if (c >= a.dv) continue;
+    if (a.splits == 1) *reinterpret_cast<uint32_t*>(a.out + orow * a.dv + c) = pack_bf16x2(acc[2 * i], acc[2 * i + 1]);
+    else *reinterpret_cast<float2*>(a.part + ((long long)split * a.T * a.Hq + orow) * a.dv + c) = make_float2(acc[2 * i], acc[2 * i + 1]);
+  }
+}
+
+// Those of a softmax warp's rows that `again` names: lanes hold their rows' m and inv.  The geometry is worked out anew: nothing of this is alive in the loops.
+template <bool kSplitP>
+__device__ __forceinline__ void fmha_rows_again(const FmArgs& a, unsigned again, int seq, int tok0, int row0, float m, float inv) {
+  const int hkv = blockIdx.y, split = blockIdx.z, q_beg = a.cu_seqlens_q[seq], q_len = a.cu_seqlens_q[seq + 1] - q_beg, ctx = a.context_lens ? a.context_lens[seq] : q_len;
+  const int n_tok = min(a.tq * a.tiles, q_beg + q_len - tok0), base_limit = a.causal ? ctx - q_len + (tok0 - q_beg) : ctx - 1;
+  const int vis_hi = a.causal ? base_limit + n_tok - 1 : base_limit, vis_lo = a.window > 0 ? max(0, base_limit - a.window + 1) : 0;
+  const int first = vis_lo / kFmBlk, total = vis_hi >= 0 ? vis_hi / kFmBlk + 1 - first : 0, per_split = (total + a.splits - 1) / a.splits;
+  const int key_lo = (first + split * per_split) * kFmBlk, key_hi = (first + min(total, (split + 1) * per_split)) * kFmBlk - 1;
+#pragma unroll 1
+  for (; again; again &= again - 1) {
+    const int l = __ffs(again) - 1, row = row0 + l, tl = (row >> 7) * a.tq + (row & 127) / a.g, limit = a.causal ? base_limit + tl : base_limit;
+    fmha_row_again<kSplitP>(a, a.paged ? a.block_tables + (long long)seq * a.bt_stride : nullptr, q_beg, hkv, tok0 + tl, hkv * a.g + (row & 127) % a.g,
+                            max(key_lo, a.window > 0 ? limit - a.window + 1 : 0), min(key_hi, limit), __shfl_sync(0xffffffffu, m, l), __shfl_sync(0xffffffffu, inv, l), split);
+  }
+}
+
 // kWG: softmax warpgroups = most tiles per CTA; kSlots: score slots of a tile
 template <int kWG, bool kSplitP, int kSlots>
 __global__ void __launch_bounds__(128 + 128 * kWG, kWG == 1 && kSlots == 2 ? 2 : 1)
 fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
-            const __grid_constant__ CUtensorMap r_map, const FmArgs a) {
+            const __grid_constant__ CUtensorMap r_map, const __grid_constant__ FmArgs a) {
   pdl_wait();                     // dependent launch: nothing above this line touches global memory
   extern __shared__ uint8_t smem_raw[];
   // swizzled tiles need 1024-byte alignment; behind static shared memory the dynamic part starts on a 16-byte boundary
@@ -402,6 +492,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
     if (have) tc_fence_after();
     __syncwarp();
     const float inv = have && l_run > 0.f ? 1.f / l_run : 0.f;
+    float all[2] = {0.f, 0.f};               // no finite number if one of the row's sums is none
 #pragma unroll 1
     for (int cblk = 0; cblk < (a.npv + 15) / 16; cblk++) {
       uint32_t o[16];
@@ -409,6 +500,8 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
       if (have) {
         tmem_ld_32x32b_x16(tmem_o + cblk * 16, o);
         tc_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) add2(all, o[j], o[j + 1]);
 #pragma unroll
         for (int j = 0; j < 16; j++) o[j] = __float_as_uint(__uint_as_float(o[j]) * inv);
       } else {
@@ -430,6 +523,9 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
         }
       }
     }
+    // rows with infinities or no numbers among their sums, whose scores are numbers
+    const unsigned again = __ballot_sync(0xffffffffu, row_ok && !(fabsf(all[0] + all[1]) < INFINITY) && l_run >= 0.f && l_run < INFINITY);
+    if (again) fmha_rows_again<kSplitP>(a, again, seq, tok0, t * 128 + wq * 32, m_run, inv);
     if (a.splits > 1 && row_ok) a.lse2[(long long)split * rows + orow] = (have && l_run > 0.f) ? m_run + log2f(l_run) : -INFINITY;
   }
 
@@ -484,6 +580,8 @@ extern "C" int ne_fmha(const void* q, long long q_ld, const void* k, long long k
   a.window = window > 0 ? window : 0; a.causal = causal; a.paged = block_tables != nullptr;
   a.block_tables = block_tables; a.bt_stride = bt_stride; a.cu_seqlens_q = cu_seqlens_q; a.context_lens = context_lens; a.num_seqs = num_seqs;
   a.scale_log2 = scale * 1.4426950408889634f; a.out = (__nv_bfloat16*)out; a.part = part; a.lse2 = lse2;
+  a.q = (const __nv_bfloat16*)q; a.k = (const __nv_bfloat16*)k; a.v = (const __nv_bfloat16*)v; a.k_rope = (const __nv_bfloat16*)k_rope;
+  a.d = D; a.k_dim = k_rope ? k_dim : D; a.q_ld = q_ld; a.r_ld = r_ld; a.k_ld = a.paged ? (long long)Hkv * D : k_ld; a.v_ld = a.paged ? (long long)Hkv * Dv : v_ld;
   CUtensorMap mq, mk, mv, mr;
   {
     uint64_t dims[3] = {(uint64_t)D, (uint64_t)Hq, (uint64_t)T}, strides[2] = {(uint64_t)D * 2, (uint64_t)q_ld * 2};

@@ -133,3 +133,51 @@ def test_a_sequence_does_not_see_its_neighbour_s_infinities():
     clean = sm100.attention_varlen(*x, cu, 0.1)
     x[:, 100:] = float("inf")
     assert torch.equal(sm100.attention_varlen(*x, cu, 0.1)[:100], clean[:100])
+
+
+def _plain(q, k, v, scale, first, window):
+    """In 64 bits, a key at a time: values of keys that a token may not see do not take part, whatever they are."""
+    s = torch.einsum("qhd,khd->hqk", q.double(), k.double()) * scale
+    at, key = torch.arange(q.shape[0], device=q.device)[:, None] + first, torch.arange(k.shape[0], device=q.device)[None, :]
+    hide = (key > at) | (key <= at - window if window else torch.zeros_like(key > at))
+    p, out = torch.softmax(s.masked_fill(hide[None], float("-inf")), -1), torch.zeros(*q.shape[:2], v.shape[2], dtype=torch.float64, device=q.device)
+    for i in range(k.shape[0]):
+        out += torch.where(hide[:, i, None, None], 0.0, p[:, :, i].t()[..., None] * v[i].double()[None])
+    return out
+
+
+# one key in the middle of a tile, of a block and of the first tile of a pair; infinities of both signs and no numbers in a few of its columns
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("kind,heads,dim,n,before,window", [("varlen", 4, 72, 300, 0, 0), ("varlen", 16, 64, 1300, 0, 0), ("paged", 4, 128, 300, 70, 100), ("paged", 4, 256, 90, 500, 130),
+                                                            ("paged", 64, 128, 400, 0, 0), ("mla", 128, 192, 300, 0, 0), ("mla", 2, 192, 200, 0, 0)])
+def test_a_value_reaches_only_the_tokens_that_see_it(kind, heads, dim, n, before, window, bad):
+    from nanoengine_b200.ops import sm100, sm100_attn
+    sm100.clear_kernel_status()
+    g = torch.Generator(device="cuda").manual_seed(7)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)             # noqa: E731
+    m, kv = n + before, 4 if heads == 64 else heads
+    q, k, v, kr = r(n, heads, dim), r(m, kv, dim), r(m, kv, 128 if kind == "mla" else dim), r(m, 64)
+    at = m - n + n // 3 + 7
+    v[at, :, 3] = bad
+    v[at + 1, :, 20] = -bad
+    cu = torch.tensor([0, n], dtype=torch.int32, device="cuda")
+    calls = sm100_attn.PROMPT_TC_CALLS[0]
+    if kind == "varlen":
+        got = sm100.attention_varlen(q, k, v, cu, dim ** -0.5, True)
+    elif kind == "mla":
+        k[:, :, 128:] = kr[:, None]
+        got = sm100.mla_prefill_ragged(q, k[:, :, :128].contiguous(), kr, v, cu, dim ** -0.5)
+    else:
+        nb = -(-m // 64)
+        kc, vc = (torch.zeros(nb + 1, 64, kv, dim, dtype=torch.bfloat16, device="cuda") for _ in "kv")
+        kc.view(-1, kv, dim)[64: 64 + m], vc.view(-1, kv, dim)[64: 64 + m] = k, v
+        bt = torch.arange(1, nb + 1, dtype=torch.int32, device="cuda")[None]
+        got = sm100_attn.gqa_attention_paged(q, kc, vc, bt, cu, torch.tensor([m], dtype=torch.int32, device="cuda"), dim ** -0.5, window)
+    assert sm100.kernel_status()[0] == 0
+    assert sm100_attn.PROMPT_TC_CALLS[0] == calls + 1
+    rep = heads // kv
+    want = _plain(q, k.repeat_interleave(rep, 1), v.repeat_interleave(rep, 1), dim ** -0.5, m - n, window)
+    fin = want.isfinite()
+    assert torch.equal(got.isfinite(), fin) and not fin.all()
+    assert torch.equal(got[~fin].nan_to_num(nan=7.0).double(), want[~fin].nan_to_num(nan=7.0, posinf=torch.finfo(torch.bfloat16).max, neginf=torch.finfo(torch.bfloat16).min))
+    assert _rel(got[fin], want[fin]) < (EXACT_P if window or dim not in (128, 192) else BF16_P)
