@@ -15,8 +15,9 @@
 // slots, which the other tile's products, or the other CTA's, fill (1063 -> 1088 us for the MLA prompts below, against issuing without the wait), PV(j-1) with
 // three (256-wide heads, nothing beside them: 177 without a wait, 197 with two slots, 186 so).
 // A barrier test costs an issuing thread 300 cycles once products are queued before it, hence an issuer per tile, and tests in threes.
-// kSplitP: probabilities stay 32-bit in effect: bf16 head and bf16 remainder (2^-17), two products against V.  Taken where the plain kernel this one
-// replaced kept them in fp32.
+// kSplitP: a probability as a bf16 head and a bf16 remainder, both rounded, so it is off by 2^-17 of itself at most, to either side, and its sum takes it whole; two
+// products against V.  Taken where the plain kernel this one replaced kept them in fp32: sums before they are rounded to bf16 are 2.7e-6 off (2-norm, 40 .. 3000
+// keys; that kernel: 1e-7 .. 8e-7, a head that is cut off: 5e-6), the results 1.66e-3, as that kernel's.
 // Shared memory: Q, then a ring of 8 KB slots (64 keys x 64 columns) shared by K and V, loaded in the order of first use; the chunks of a block's K
 // or V (a group) share one barrier.
 // Rows of V in front of the window or past the last visible key (pages that belong to nobody, rows of the next sequence: often no numbers) are zeroed in shared
@@ -448,10 +449,10 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
         if constexpr (kSplitP) {
           uint32_t lo[16];
 #pragma unroll
-          for (int j = 0; j < 16; j++) {       // the head is cut off, not rounded: the remainder takes the difference either way
-            hi[j] = __byte_perm(x[2 * j], x[2 * j + 1], 0x7632);
+          for (int j = 0; j < 16; j++) {
+            hi[j] = pack_bf16x2(__uint_as_float(x[2 * j]), __uint_as_float(x[2 * j + 1]));
             add2(ps, x[2 * j], x[2 * j + 1]);
-            lo[j] = pack_bf16x2(__uint_as_float(x[2 * j]) - __uint_as_float(x[2 * j] & 0xffff0000u), __uint_as_float(x[2 * j + 1]) - __uint_as_float(x[2 * j + 1] & 0xffff0000u));
+            lo[j] = pack_bf16x2(__uint_as_float(x[2 * j]) - __uint_as_float(hi[j] << 16), __uint_as_float(x[2 * j + 1]) - __uint_as_float(hi[j] & 0xffff0000u));
           }
           tmem_st_32x32b_x16(ts + 32 + c * 16, lo);
         } else {

@@ -5,7 +5,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-# results are bf16 (2^-9 / sqrt(3) = 1.1e-3 in the 2-norm, at most 2^-8 of a value); probabilities enter as two bf16 terms, 2^-17 each
+# results are bf16 (2^-9 / sqrt(3) = 1.1e-3 in the 2-norm, at most 2^-8 of a value); probabilities enter as two bf16 terms, 2^-17 of them left out
 EXACT_P = 2e-3
 BF16_P = 1e-2           # D = 128 without a window: probabilities in bf16
 
@@ -181,3 +181,23 @@ def test_a_value_reaches_only_the_tokens_that_see_it(kind, heads, dim, n, before
     assert torch.equal(got.isfinite(), fin) and not fin.all()
     assert torch.equal(got[~fin].nan_to_num(nan=7.0).double(), want[~fin].nan_to_num(nan=7.0, posinf=torch.finfo(torch.bfloat16).max, neginf=torch.finfo(torch.bfloat16).min))
     assert _rel(got[fin], want[fin]) < (EXACT_P if window or dim not in (128, 192) else BF16_P)
+
+
+@pytest.mark.parametrize("dim,window,m,n", [(72, 0, 40, 40), (128, 70, 300, 90), (256, 0, 500, 130)])
+def test_probabilities_keep_17_bits(dim, window, m, n):
+    """The kernel's 32-bit slices: a probability is off by 2^-17 of itself at most, the rest is 32-bit sums and an exponential (2^-20 is a bound for both)."""
+    from nanoengine_b200.ops import sm100_attn
+    g = torch.Generator(device="cuda").manual_seed(8)
+    hq, hkv, nb = 8, 2, -(-m // 64)
+    k, v = (torch.randn(nb, 64, hkv, dim, generator=g, device="cuda").to(torch.bfloat16) for _ in "kv")
+    q = (2 * torch.randn(n, hq, dim, generator=g, device="cuda")).to(torch.bfloat16)
+    bt, cu, cl = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([list(range(nb))], [0, n], [m]))
+    part, lse = torch.empty(2, n, hq, dim, device="cuda"), torch.empty(2, n, hq, device="cuda")
+    p = lambda t: t.data_ptr()             # noqa: E731
+    assert sm100_attn._fmha_call()(p(q), q.stride(0), p(k), k.stride(0), dim, 0, 0, p(v), v.stride(0), nb, p(bt), nb, p(cu), p(cl), 1, n, hq, hkv, dim, dim, 1, n // 32 + 1, 2, window, 1,
+                                   dim ** -0.5, 1, 0, p(part), p(lse), torch.cuda.current_stream().cuda_stream) == 0
+    w = torch.exp2(lse.double() - lse.double().amax(0))
+    got = (w / w.sum(0))[..., None] * part.double()
+    kk, vv = (x.reshape(-1, hkv, dim)[:m] for x in (k, v))
+    want, size = _attend(q, kk, vv, dim ** -0.5, m - n, window), _attend(q, kk, vv.abs(), dim ** -0.5, m - n, window)
+    assert ((got.sum(0) - want).abs() / size).max().item() < 2 ** -17 + 2 ** -20
