@@ -527,7 +527,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
     // rows with infinities or no numbers among their sums, whose scores are numbers
     const unsigned again = __ballot_sync(0xffffffffu, row_ok && !(fabsf(all[0] + all[1]) < INFINITY) && l_run >= 0.f && l_run < INFINITY);
     if (again) fmha_rows_again<kSplitP>(a, again, seq, tok0, t * 128 + wq * 32, m_run, inv);
-    if (a.splits > 1 && row_ok) a.lse2[(long long)split * rows + orow] = (have && l_run > 0.f) ? m_run + log2f(l_run) : -INFINITY;
+    if (a.splits > 1 && row_ok) a.lse2[(long long)split * rows + orow] = (have && l_run != 0.f) ? m_run + log2f(l_run) : -INFINITY;      // no number: the merge passes it on
   }
 
   tc_fence_before();

@@ -201,3 +201,15 @@ def test_probabilities_keep_17_bits(dim, window, m, n):
     kk, vv = (x.reshape(-1, hkv, dim)[:m] for x in (k, v))
     want, size = _attend(q, kk, vv, dim ** -0.5, m - n, window), _attend(q, kk, vv.abs(), dim ** -0.5, m - n, window)
     assert ((got.sum(0) - want).abs() / size).max().item() < 2 ** -17 + 2 ** -20
+
+
+@pytest.mark.parametrize("dim,window,n", [(256, 0, 3), (128, 900, 40), (72, 0, 1)])
+def test_a_score_that_is_no_number_shows_through_slices(dim, window, n):
+    from nanoengine_b200.ops import sm100_attn
+    hq, hkv, m = 8, 2, 2000
+    kc, vc = (torch.randn(32, 64, hkv, dim, device="cuda").to(torch.bfloat16) for _ in "kv")
+    q = torch.randn(n, hq, dim, device="cuda").to(torch.bfloat16)
+    kc[(m - n // 2 - 500) // 64, (m - n // 2 - 500) % 64, 1] = float("nan")                # of one key, in one of the slices, for the second half of the heads
+    bt, cu, cl = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([list(range(32))], [0, n], [m]))
+    got = sm100_attn.gqa_attention_paged(q, kc, vc, bt, cu, cl, dim ** -0.5, window)
+    assert got[:, : hq // 2].isfinite().all() and got[:, hq // 2:].isnan().all()
