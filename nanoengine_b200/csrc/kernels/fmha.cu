@@ -83,6 +83,9 @@ __device__ __forceinline__ void mbar_test3(uint32_t a, uint32_t pa, uint32_t b, 
   ra = x; rb = y; rc = z;
 }
 
+// tokens of a sequence; those past the tensors' end are none of its rows (n_tok), nor keys where they are the tokens themselves
+__device__ __forceinline__ int fm_len(const FmArgs& a, int seq, int beg) { return (a.context_lens ? a.cu_seqlens_q[seq + 1] : min(a.cu_seqlens_q[seq + 1], a.T)) - beg; }
+
 // sum of a[i] b[i], n a multiple of 8, both on 16-byte boundaries
 __device__ __forceinline__ float fm_dot(const __nv_bfloat16* a, const __nv_bfloat16* b, int n) {
   float s = 0.f;
@@ -156,8 +159,8 @@ __device__ __forceinline__ void fmha_row_again(const FmArgs& a, const int* bt, i
 // Those of a softmax warp's rows that `again` names: lanes hold their rows' m and inv.  The geometry is worked out anew: nothing of this is alive in the loops.
 template <bool kSplitP>
 __device__ __forceinline__ void fmha_rows_again(const FmArgs& a, unsigned again, int seq, int tok0, int row0, float m, float inv) {
-  const int hkv = blockIdx.y, split = blockIdx.z, q_beg = a.cu_seqlens_q[seq], q_len = a.cu_seqlens_q[seq + 1] - q_beg, ctx = a.context_lens ? a.context_lens[seq] : q_len;
-  const int n_tok = min(a.tq * a.tiles, q_beg + q_len - tok0), base_limit = a.causal ? ctx - q_len + (tok0 - q_beg) : ctx - 1;
+  const int hkv = blockIdx.y, split = blockIdx.z, q_beg = a.cu_seqlens_q[seq], q_len = fm_len(a, seq, q_beg), ctx = a.context_lens ? a.context_lens[seq] : q_len;
+  const int n_tok = min(a.tq * a.tiles, min(q_beg + q_len, a.T) - tok0), base_limit = a.causal ? ctx - q_len + (tok0 - q_beg) : ctx - 1;
   const int vis_hi = a.causal ? base_limit + n_tok - 1 : base_limit, vis_lo = a.window > 0 ? max(0, base_limit - a.window + 1) : 0;
   const int first = vis_lo / kFmBlk, total = vis_hi >= 0 ? vis_hi / kFmBlk + 1 - first : 0, per_split = (total + a.splits - 1) / a.splits;
   const int key_lo = (first + split * per_split) * kFmBlk, key_hi = (first + min(total, (split + 1) * per_split)) * kFmBlk - 1;
@@ -205,8 +208,8 @@ fmha_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ C
   // geometry (uniform over the CTA)
   int nt = 1, nblk = 0, blk0 = 0, n_tok = 0, base_limit = -1, vis_lo = 0, vis_hi = -1, k_beg = 0;
   if (seq >= 0) {
-    const int q_beg = a.cu_seqlens_q[seq], q_len = a.cu_seqlens_q[seq + 1] - q_beg, ctx = a.context_lens ? a.context_lens[seq] : q_len;
-    n_tok = min(a.tq * a.tiles, q_beg + q_len - tok0);
+    const int q_beg = a.cu_seqlens_q[seq], q_len = fm_len(a, seq, q_beg), ctx = a.context_lens ? a.context_lens[seq] : q_len;
+    n_tok = min(a.tq * a.tiles, min(q_beg + q_len, a.T) - tok0);
     nt = n_tok > a.tq ? 2 : 1;
     k_beg = q_beg;
     base_limit = a.causal ? ctx - q_len + (tok0 - q_beg) : ctx - 1;          // last key visible to the tile's first token

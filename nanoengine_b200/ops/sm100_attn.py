@@ -395,6 +395,7 @@ def attention_varlen(q, k, v, cu_seqlens, scale, causal: bool = False):
     if T == 0:
         return torch.empty(T, H, D, dtype=torch.bfloat16, device=q.device)
     cu = _i32(cu_seqlens)
+    assert cu.device == q.device and cu.numel() > 1, "sequence boundaries on the GPU, of one sequence at least"
     if scale > 0 and _fmha_covers(1, D, D) and k.shape == q.shape and v.shape == q.shape:
         return _fmha(*[t if _rows16(t) else t.clone(memory_format=torch.contiguous_format) for t in (q, k, v)], cu, scale, causal, True)
     k, v = k.contiguous(), v.contiguous()

@@ -213,3 +213,22 @@ def test_a_score_that_is_no_number_shows_through_slices(dim, window, n):
     bt, cu, cl = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([list(range(32))], [0, n], [m]))
     got = sm100_attn.gqa_attention_paged(q, kc, vc, bt, cu, cl, dim ** -0.5, window)
     assert got[:, : hq // 2].isfinite().all() and got[:, hq // 2:].isnan().all()
+
+
+def test_boundaries_past_the_tensors_end_write_nothing_there():
+    """Rows and keys end with the tensors, whatever the boundaries say (the buffers of this test are longer, so that nothing can fault); those on the host are refused."""
+    from nanoengine_b200.ops import sm100, sm100_attn
+    t, more, h, dim = 150, 300, 4, 72
+    q, k, v = (torch.randn(more, h, dim, device="cuda").to(torch.bfloat16) for _ in "qkv")
+    p = lambda x: x.data_ptr()             # noqa: E731
+    for causal in (0, 1):
+        out = torch.full((more, h, dim), 5.0, dtype=torch.bfloat16, device="cuda")
+        cu = torch.tensor([0, 100, 290], dtype=torch.int32, device="cuda")
+        assert sm100_attn._fmha_call()(p(q), q.stride(0), p(k), k.stride(0), dim, 0, 0, p(v), v.stride(0), t, 0, 0, p(cu), 0, 2, t, h, h, dim, dim, 1, 4, 1, 0, causal, 0.1, 1, p(out), 0, 0,
+                                       torch.cuda.current_stream().cuda_stream) == 0
+        assert (out[t:] == 5.0).all()
+        cu[2] = t
+        assert torch.equal(out[:t], sm100.attention_varlen(q[:t], k[:t], v[:t], cu, 0.1, bool(causal)))
+    for cu in (torch.tensor([0, t], dtype=torch.int32), torch.tensor([0], dtype=torch.int32, device="cuda")):
+        with pytest.raises(AssertionError):
+            sm100.attention_varlen(q[:t], k[:t], v[:t], cu, 0.1)
