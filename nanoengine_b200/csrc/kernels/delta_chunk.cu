@@ -11,7 +11,7 @@
 //   scan     one CTA per (sequence, head, 32 of the 128 value columns - columns are independent of each other given T and P T -) walks the chunks with its
 //            part of the state in registers.  Four short products in a row per chunk, 32 x 128 x 128 and smaller, each waiting for the one before.
 // A 32-bit operand enters a product as three bf16 terms (x = h + m + l to 2^-25); k and q are bf16 already and enter once, so K S^T and U^T K take three
-// products, T R six.  Outputs, which are rounded to bf16 behind the norm, are content with two terms of P T.
+// products, T R and P T R six.
 // Warp-level mma.sync and not tcgen05: S, R and U change between accumulator and operand three times a chunk, which here is a pack in registers (the
 // accumulator of a transposed product has the layout of the next product's A operand) and one exchange through shared memory, without the trip through
 // TMEM, the descriptor tiles and a commit for each.
@@ -20,7 +20,8 @@
 //
 // Bound: the matrix instructions of the scan (190 a chunk and warp, 8 cycles each on a scheduler: 3,000 cycles for 64 tokens x 32 columns, beside as many of
 // shared memory), and its chain of products.  Measured: 4 prompts of 750 .. 2250 tokens, 32 heads over 16: 14774 us as batched fp32 products and triangular
-// solves of a library per sequence, 580 us so (prepare 172, scan 352, norm 53).  Error of the final state against 64 bits 1.7e-7 (before: 1.8e-7).
+// solves of a library per sequence, 571 us so.  Errors against 64 bits: final states 1.8e-7 (before: 1.8e-7), outputs in front of the norm 4.3e-7 (3.6e-6 with two
+// terms of P T and of R).
 //
 // Replaces in the reference: the chunked prefill of triton/fla (layers/backends/delta_net/components/recurrence.py:100-200).
 #include "ptx.cuh"
@@ -33,7 +34,7 @@ constexpr int kDcC = 64;                       // tokens per chunk
 constexpr int kDcD = 128;                      // key and value size
 constexpr int kDcThreads = 256;
 constexpr int kDcPairs = 10;                   // (row block j, column block i <= j) of 16 x 16 of a lower triangular 64 x 64
-constexpr int kDcFragBytes = kDcPairs * (3 + 2) * 512;      // T in three terms, P T in two; 512 bytes: 16 x 16 as the B operands of two mma (16 B per lane)
+constexpr int kDcFragBytes = kDcPairs * 2 * 3 * 512;        // T and P T in three terms; 512 bytes: 16 x 16 as the B operands of two mma (16 B per lane)
 
 struct DcArgs {
   const __nv_bfloat16* q; const __nv_bfloat16* k; const __nv_bfloat16* v; long long qk_ld, v_ld;
@@ -262,10 +263,9 @@ __global__ void __launch_bounds__(kDcThreads, 3) delta_chunk_prepare_kernel(cons
         const float2 f = *reinterpret_cast<const float2*>(src + n * 8 * kDcLd + r * 8);
         split3(f.x, f.y, w[0][n * 2 + r], w[1][n * 2 + r], w[2][n * 2 + r]);
       }
-    uint4* dst = reinterpret_cast<uint4*>(frag + (pt ? kDcPairs * 3 + p * 2 : p * 3) * 512) + lane;
-    dst[0] = make_uint4(w[0][0], w[0][1], w[0][2], w[0][3]);
-    dst[32] = make_uint4(w[1][0], w[1][1], w[1][2], w[1][3]);
-    if (!pt) dst[64] = make_uint4(w[2][0], w[2][1], w[2][2], w[2][3]);
+    uint4* dst = reinterpret_cast<uint4*>(frag + i * 3 * 512) + lane;
+#pragma unroll
+    for (int t = 0; t < 3; t++) dst[32 * t] = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
   }
   if (tid < kDcC) {
     const float e = expf((float)s_g[tid]), b = s_b[tid];
@@ -291,7 +291,8 @@ __global__ void __launch_bounds__(kDcThreads, 2) delta_chunk_scan_kernel(const D
   if (n < a.min_n || n <= 0) return;
   const int st_slot = a.slots[seq];
   if (!NE_INDEX_OK(st_slot, BK_STATE_SLOTS, kKernelDc, __LINE__)) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, j = warp & 3, g = lane >> 2, c2 = (lane & 3) * 2;
+  // j: the warp's 16 tokens of a chunk; row block j of T or P T has j + 1 products, so a scheduler's two warps (w and w + 4) take j and 3 - j (600 -> 571 us)
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, j = warp < 4 ? warp : 7 - warp, g = lane >> 2, c2 = (lane & 3) * 2;
   int chunk0 = 0;             // chunks of the sequences in front
   for (int s0 = lane; s0 < seq; s0 += 32) chunk0 += (a.cu[s0 + 1] - a.cu[s0] + kDcC - 1) / kDcC;
   chunk0 = __reduce_add_sync(0xffffffffu, chunk0);
@@ -355,9 +356,7 @@ __global__ void __launch_bounds__(kDcThreads, 2) delta_chunk_scan_kernel(const D
     for (int kt = 0; kt < 4; kt++)
       if (kt <= j)
 #pragma unroll
-        for (int t = 0; t < 3; t++)
-          if (t < 2 || warp < 4)
-            fb[kt][t] = __ldg(reinterpret_cast<const uint4*>(frag + (warp < 4 ? dc_pair(j, kt) * 3 + t : kDcPairs * 3 + dc_pair(j, kt) * 2 + t) * 512) + lane);
+        for (int t = 0; t < 3; t++) fb[kt][t] = __ldg(reinterpret_cast<const uint4*>(frag + (((warp < 4 ? 0 : kDcPairs) + dc_pair(j, kt)) * 3 + t) * 512) + lane);
     // ---- S K^T and S Q^T: columns = this warp's 16 tokens
     float D[kDcM][2][4] = {};
 #pragma unroll
@@ -393,27 +392,27 @@ __global__ void __launch_bounds__(kDcThreads, 2) delta_chunk_scan_kernel(const D
       }
     if (warp < 4) put(sR, j, D);
     __syncthreads();          // R is there; nobody reads the state's fragments any more
-    // ---- U = T R, O += P T R
-    if (warp < 4) {
-      float U[kDcM][2][4] = {};
+    // ---- U = T R (outputs: P T R)
+    float U[kDcM][2][4] = {};
 #pragma unroll
-      for (int kt = 0; kt < 4; kt++) {
-        if (kt > j) continue;
+    for (int kt = 0; kt < 4; kt++) {
+      if (kt > j) continue;
 #pragma unroll
-        for (int m = 0; m < kDcM; m++) {
-          uint32_t f[3][4];
+      for (int m = 0; m < kDcM; m++) {
+        uint32_t f[3][4];
 #pragma unroll
-          for (int t = 0; t < 3; t++) get(sR, kt, m, t, f[t]);
-          // smallest products first
+        for (int t = 0; t < 3; t++) get(sR, kt, m, t, f[t]);
+        // smallest products first
 #pragma unroll
-          for (int s = 2; s >= 0; s--)
+        for (int s = 2; s >= 0; s--)
 #pragma unroll
-            for (int t = 0; t <= s; t++) {
-              mma_bf16(U[m][0], f[t], fb[kt][s - t].x, fb[kt][s - t].y);
-              mma_bf16(U[m][1], f[t], fb[kt][s - t].z, fb[kt][s - t].w);
-            }
-        }
+          for (int t = 0; t <= s; t++) {
+            mma_bf16(U[m][0], f[t], fb[kt][s - t].x, fb[kt][s - t].y);
+            mma_bf16(U[m][1], f[t], fb[kt][s - t].z, fb[kt][s - t].w);
+          }
       }
+    }
+    if (warp < 4) {
 #pragma unroll
       for (int x = 0; x < 2; x++)
 #pragma unroll
@@ -425,17 +424,11 @@ __global__ void __launch_bounds__(kDcThreads, 2) delta_chunk_scan_kernel(const D
       put(sS, j, U);
     } else {
 #pragma unroll
-      for (int kt = 0; kt < 4; kt++) {
-        if (kt > j) continue;
+      for (int m = 0; m < kDcM; m++)
 #pragma unroll
-        for (int m = 0; m < kDcM; m++) {
-          uint32_t f[2][4];
-          get(sR, kt, m, 0, f[0]); get(sR, kt, m, 1, f[1]);
-          mma_bf16(D[m][0], f[1], fb[kt][0].x, fb[kt][0].y); mma_bf16(D[m][1], f[1], fb[kt][0].z, fb[kt][0].w);
-          mma_bf16(D[m][0], f[0], fb[kt][1].x, fb[kt][1].y); mma_bf16(D[m][1], f[0], fb[kt][1].z, fb[kt][1].w);
-          mma_bf16(D[m][0], f[0], fb[kt][0].x, fb[kt][0].y); mma_bf16(D[m][1], f[0], fb[kt][0].z, fb[kt][0].w);
-        }
-      }
+        for (int x = 0; x < 2; x++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) D[m][x][e] += U[m][x][e];
     }
     __syncthreads();          // U is there
     // ---- S = e^(G_C) S + (e^(G_C - G) U)^T K

@@ -94,3 +94,22 @@ def test_decay_per_channel(heads, lens, bound, scale):
     want = want * torch.rsqrt(want.square().mean(-1, keepdim=True) + 1e-6) * w.double() * torch.sigmoid(z.double())
     assert sm100.kernel_status()[0] == 0
     assert _rel(got.view(t, heads, D), want) < OUT and _rel(state, want_state) < STATE
+
+
+@pytest.mark.parametrize("lens", [[64], [200, 64, 5, 129]])
+@pytest.mark.parametrize("alike", [0.0, 0.99])
+def test_outputs_in_front_of_the_norm_are_32_bit(lens, alike, monkeypatch):
+    """`alike`: every key is mostly the same vector, where the inverse of a chunk's system has the largest entries (its products of two rows are 0.98, its decay 0.999)."""
+    from nanoengine_b200.ops import sm100
+    hk, hv = 2, 4
+    gen, r, q, k, v, state, slots, fresh, cu, z, w = _inputs(lens, hk, hv, 9)
+    t = sum(lens)
+    k.copy_((alike * r(1, hk, D) + (1 - alike ** 2) ** 0.5 * r(t, hk, D)).to(torch.bfloat16))
+    a, b = r(t, 2 * hv).to(torch.bfloat16).split(hv, 1)
+    A, bias = torch.full((hv,), 0.001, device="cuda").log(), torch.zeros(hv, device="cuda")
+    g = -A.double().exp() * torch.nn.functional.softplus(a.double() + bias.double())
+    want, want_state = _oracle(_unit(q, hv // hk, D ** -0.5), _unit(k, hv // hk), v.double(), g, torch.sigmoid(b.double()), state, fresh.tolist(), lens, slots.tolist())
+    seen, norm = [], sm100.rmsnorm_gated
+    monkeypatch.setattr(sm100, "rmsnorm_gated", lambda x, *rest: (seen.append(x.clone()), norm(x, *rest))[1])
+    sm100.gdn_recurrent(q, k, v, a, b, A, bias, state, slots, torch.tensor(cu, dtype=torch.int32, device="cuda"), fresh, z, w, 1e-6, max(lens), cu)
+    assert len(seen) == 1 and _rel(seen[0], want) < STATE and _rel(state, want_state) < STATE
