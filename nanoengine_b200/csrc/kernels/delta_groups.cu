@@ -93,7 +93,6 @@ __global__ void __launch_bounds__(kDgThreads, 3) delta_groups_kernel(const DgArg
       if (have) x = *reinterpret_cast<const ulonglong2*>(Sg + r * 4 * 128 + i * 32);
       S[r][2 * i] = x.x; S[r][2 * i + 1] = x.y;
     }
-  if (tid < 16) s_P[tid >> 2][tid & 3] = make_float4(0.f, 0.f, 0.f, 0.f);
   const float expA = expf(a.A_log[h]);
   float bias[kVec ? 4 : 1];
 #pragma unroll
@@ -255,6 +254,11 @@ __global__ void __launch_bounds__(kDgThreads, 3) delta_groups_kernel(const DgArg
         for (int s = 0; s < t; s++) y = fmaf(-s_A[gi][t * (t - 1) / 2 + s], u[s], y);
         u[t] = y * s_beta[gi * 4 + t];
       }
+      if (gi * 4 + 4 > m) {
+#pragma unroll
+        for (int t = 1; t < 4; t++)
+          if (gi * 4 + t >= m) u[t] = 0.f;     // behind the end: nothing, whatever the state holds
+      }
       reduce16(x, sub, w);
 #pragma unroll
       for (int i = 0; i < 4; i++) {
@@ -278,7 +282,13 @@ __global__ void __launch_bounds__(kDgThreads, 3) delta_groups_kernel(const DgArg
       for (int e = 0; e < 2; e++) {
         const int t = (sub >> 2) * 2 + e;
         const float4 p = s_P[gi][t];
-        const float o = fmaf(p.w, u[3], fmaf(p.z, u[2], fmaf(p.y, u[1], fmaf(p.x, u[0], w[e]))));
+        float o = fmaf(p.x, u[0], w[e]);
+        if (e == 1) o = fmaf(p.y, u[1], o);
+        if (sub & 4) {                         // later tokens by a choice, not by a factor of zero: their u may be no number
+          if (e == 0) o = fmaf(p.y, u[1], o);
+          o = fmaf(p.z, u[2], o);
+          if (e == 1) o = fmaf(p.w, u[3], o);
+        }
         if (gi * 4 + t < m) out[(long long)(gi * 4 + t) * a.H * 128] = o;
       }
     }

@@ -113,3 +113,47 @@ def test_outputs_in_front_of_the_norm_are_32_bit(lens, alike, monkeypatch):
     monkeypatch.setattr(sm100, "rmsnorm_gated", lambda x, *rest: (seen.append(x.clone()), norm(x, *rest))[1])
     sm100.gdn_recurrent(q, k, v, a, b, A, bias, state, slots, torch.tensor(cu, dtype=torch.int32, device="cuda"), fresh, z, w, 1e-6, max(lens), cu)
     assert len(seen) == 1 and _rel(seen[0], want) < STATE and _rel(state, want_state) < STATE
+
+
+@pytest.mark.parametrize("what", ["v", "k", "q", "gate", "beta"])
+@pytest.mark.parametrize("per_channel", [False, True])
+@pytest.mark.parametrize("at", range(8, 13))
+def test_a_token_that_is_no_number_leaves_the_earlier_ones_alone(per_channel, what, at):
+    from nanoengine_b200.ops import sm100
+    heads, lens = 2, [at + 1 if at == 12 else 15, 9]
+    gen, r, q, k, v, state, slots, fresh, cu, z, w = _inputs(lens, heads, heads, 10)
+    t = sum(lens)
+    a, b = r(t, heads * (D if per_channel else 1)).to(torch.bfloat16), r(t, heads).to(torch.bfloat16)
+    A, bias = torch.zeros(heads, device="cuda"), torch.zeros(heads * (D if per_channel else 1), device="cuda")
+    cu = torch.tensor(cu, dtype=torch.int32, device="cuda")
+
+    def run(st):
+        if per_channel:
+            return sm100.kda_recurrent(q, k, v, a, b, A, bias, None, st, slots, cu, fresh, z, w, 1e-6).view(t, heads, D)
+        return sm100.gdn_recurrent(q, k, v, a, b, A, bias, st, slots, cu, fresh, z, w, 1e-6, max(lens)).view(t, heads, D)
+
+    st, clean = state.clone(), run(clean_state := state.clone())
+    {"v": v, "k": k, "q": q, "gate": a.view(t, heads, -1), "beta": b.view(t, heads, 1)}[what][at, 1] = float("nan")
+    got = run(st)
+    hit = torch.zeros(t, heads, dtype=torch.bool, device="cuda")
+    hit[at: at + 1 if what == "q" else lens[0], 1] = True                 # a query is its token's alone, the others stay in the state
+    assert got[hit].isnan().all() and torch.equal(got[~hit], clean[~hit])
+    assert torch.equal(st[slots[1].long()], clean_state[slots[1].long()]) and torch.equal(st[slots[0].long(), 0], clean_state[slots[0].long(), 0])
+
+
+@pytest.mark.parametrize("per_channel", [False, True])
+def test_an_infinite_state_row_is_not_worked_on_behind_the_end(per_channel):
+    from nanoengine_b200.ops import sm100
+    heads, n = 1, 9
+    gen, r, q, k, v, state, slots, fresh, cu, z, w = _inputs([n], heads, heads, 11)
+    a, b = r(n, heads * (D if per_channel else 1)).to(torch.bfloat16), r(n, heads).to(torch.bfloat16)
+    A, bias = torch.zeros(heads, device="cuda"), torch.zeros(heads * (D if per_channel else 1), device="cuda")
+    v[n - 1, 0, 5] = float("inf")                                         # the last token's write: its row of the state is infinite, of the signs of its key
+    cu = torch.tensor(cu, dtype=torch.int32, device="cuda")
+    if per_channel:
+        sm100.kda_recurrent(q, k, v, a, b, A, bias, None, state, slots, cu, fresh, z, w, 1e-6)
+    else:
+        sm100.gdn_recurrent(q, k, v, a, b, A, bias, state, slots, cu, fresh, z, w, 1e-6, n)
+    row = state[slots[0].long(), 0, 5]
+    assert torch.equal(row, torch.where(k[n - 1, 0] > 0, float("inf"), float("-inf")))
+    assert state[slots[0].long(), 0, :5].isfinite().all() and state[slots[0].long(), 0, 6:].isfinite().all()
