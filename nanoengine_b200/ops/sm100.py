@@ -1067,7 +1067,7 @@ def hisparse_writeback(hot: torch.Tensor, cold: torch.Tensor, new_slot: torch.Te
 
 # ---- gated delta-net linear attention ---------------------------------------------------------------
 def _i32(t):
-    return t if t.dtype == torch.int32 else t.int()
+    return (t if t.dtype == torch.int32 else t.int()).contiguous()
 
 
 def gdn_conv(x: torch.Tensor, weight: torch.Tensor, conv_state: torch.Tensor, slots: torch.Tensor, cu_seqlens: torch.Tensor,
@@ -1142,6 +1142,9 @@ def gdn_recurrent(q, k, v, a, b, A_log, dt_bias, state, slots, cu_seqlens, fresh
     assert q.stride(0) == k.stride(0) and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.stride(0) == b.stride(0)
     assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (Hv, Dv, Dk)
     assert A_log.dtype == torch.float32 and dt_bias.dtype == torch.float32 and norm_w.dtype == torch.bfloat16
+    if a.stride(1) != 1 or b.stride(1) != 1:
+        a, b = a.contiguous(), b.contiguous()
+    A_log, dt_bias, norm_w = A_log.contiguous(), dt_bias.contiguous(), norm_w.contiguous()
     out = torch.empty(T, Hv, Dv, dtype=torch.bfloat16, device=q.device)
     slots, cu, fresh = _i32(slots), _i32(cu_seqlens), _i32(fresh)
     skip = 1 << 30

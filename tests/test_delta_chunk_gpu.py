@@ -157,3 +157,20 @@ def test_an_infinite_state_row_is_not_worked_on_behind_the_end(per_channel):
     row = state[slots[0].long(), 0, 5]
     assert torch.equal(row, torch.where(k[n - 1, 0] > 0, float("inf"), float("-inf")))
     assert state[slots[0].long(), 0, :5].isfinite().all() and state[slots[0].long(), 0, 6:].isfinite().all()
+
+
+@pytest.mark.parametrize("lens", [[2, 3], [9, 30], [70, 3, 129], [200]])
+def test_strided_gates_and_tables(lens):
+    from nanoengine_b200.ops import sm100
+    hk, hv = 1, 2
+    gen, r, q, k, v, state, slots, fresh, cu, z, w = _inputs(lens, hk, hv, 12)
+    t, n = sum(lens), len(lens)
+    ab = r(t, hv, 2).to(torch.bfloat16)
+    A, bias, w2 = r(hv, 3) * 0.3, r(hv, 3), torch.stack([w, -w], 1)
+    table = torch.stack([slots, fresh, torch.tensor(cu[1:], dtype=torch.int32, device="cuda")], 1)         # a row per sequence
+    ends = torch.stack([torch.tensor(cu, dtype=torch.int32, device="cuda"), torch.zeros(n + 1, dtype=torch.int32, device="cuda")], 1)
+    one, two = state.clone(), state.clone()
+    want = sm100.gdn_recurrent(q, k, v, ab[..., 0].contiguous(), ab[..., 1].contiguous(), A[:, 1].contiguous(), bias[:, 2].contiguous(), one, slots, ends[:, 0].contiguous(), fresh, z, w,
+                               1e-6, max(lens), cu)
+    got = sm100.gdn_recurrent(q, k, v, ab[..., 0], ab[..., 1], A[:, 1], bias[:, 2], two, table[:, 0], ends[:, 0], table[:, 1], z, w2[:, 0], 1e-6, max(lens), cu)
+    assert torch.equal(got, want) and torch.equal(one, two)
