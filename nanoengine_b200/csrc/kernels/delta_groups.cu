@@ -10,8 +10,8 @@
 // the 16 scalars of a group are made by one warp, sixteen tokens (four groups) at a time, in shared memory; their rows arrive by asynchronous copies while the
 // sixteen before are worked on.  A reduction leaves every lane with its share of the sums (14 exchanges for 16 sums, not 48).
 // FMA pipe and shared memory are needed about equally (832 cycles a group and head half on an SM each).  Measured: per channel, 6 prompts of 500 .. 1500
-// tokens, 32 heads: 2690 -> 1060 us (before: gdn.cu's kernel, token by token, 40 exchanges of a whole warp a token); error of the final state against 64 bits
-// 2.8e-7 (before: 8.8e-7).  Per head from 64 tokens on delta_chunk.cu has the smaller error and, from 300, the shorter time.
+// tokens, 32 heads: 2690 -> 926 us (before: gdn.cu's kernel, token by token, 40 exchanges of a whole warp a token); error of the final state against 64 bits
+// 2.2e-7 (before: 8.8e-7).  Per head from 64 tokens on delta_chunk.cu has the smaller error and, from 300, the shorter time.
 //
 // Replaces in the reference: layers/backends/delta_net/kda.py:300-377.
 #include "ptx.cuh"
@@ -28,7 +28,7 @@ struct DgArgs {
   long long qk_ld, v_ld, g_ld, b_ld;           // g: [T, H, 128] contiguous (per channel) or rows of at least H
   const float* A_log; const float* dt_bias; float lower_bound;
   float* state; const int* slots; const int* cu; const int* fresh; float* raw;
-  int B, H, rep, max_n;
+  int B, H, rep, min_n, max_n;
 };
 
 __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
@@ -56,29 +56,14 @@ __device__ __forceinline__ void reduce16(const float (&x)[4][4], int sub, float 
   for (int t = 0; t < 2; t++) w[t] = (sub & 1 ? z[t][1] : z[t][0]) + __shfl_xor_sync(0xffffffffu, sub & 1 ? z[t][0] : z[t][1], 1);
 }
 
+// blockIdx.x's half head of a sequence
 template <bool kVec>
-__global__ void __launch_bounds__(kDgThreads, 3) delta_groups_kernel(const DgArgs a) {
-  pdl_wait(); pdl_trigger();
-  extern __shared__ __align__(16) uint8_t smem_raw[];
+__device__ __forceinline__ void delta_groups_sequence(const DgArgs& a, int seq, uint8_t* smem_raw) {
   __shared__ float s_beta[kDgTok], s_A[4][8];
   __shared__ float4 s_P[4][4];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, grp = lane >> 3, sub = lane & 7;
-  // sequences in the order of their lengths, longest first: this CTA's is the one with blockIdx.y longer (or equal and earlier) ones
-  int seq = a.B > 64 ? (int)blockIdx.y : -1;
-  for (int s0 = 0; s0 < a.B && seq < 0; s0 += 32) {
-    const int s = s0 + lane;
-    int rank = -1;
-    if (s < a.B) {
-      const int n = a.cu[s + 1] - a.cu[s];
-      rank = 0;
-      for (int x = 0; x < a.B; x++) { const int nx = a.cu[x + 1] - a.cu[x]; rank += nx > n || (nx == n && x < s); }
-    }
-    const unsigned hit = __ballot_sync(0xffffffffu, rank == (int)blockIdx.y);
-    if (hit) seq = s0 + __ffs(hit) - 1;
-  }
   const int h = blockIdx.x >> 1, row0 = (blockIdx.x & 1) * kDgRows, hk = h / a.rep;
   const int start = a.cu[seq], n = a.cu[seq + 1] - start;
-  if (n <= 0 || n >= a.max_n) return;
   const int slot = a.slots[seq];
   if (!NE_INDEX_OK(slot, BK_STATE_SLOTS, 28, __LINE__)) return;
   // lane: rows row0 + warp 16 + r 4 + grp, columns i 32 + sub 4 ..
@@ -299,23 +284,88 @@ __global__ void __launch_bounds__(kDgThreads, 3) delta_groups_kernel(const DgArg
     for (int i = 0; i < 4; i++) *reinterpret_cast<ulonglong2*>(Sg + r * 4 * 128 + i * 32) = make_ulonglong2(S[r][2 * i], S[r][2 * i + 1]);
 }
 
+template <bool kVec>
+__global__ void __launch_bounds__(kDgThreads, 3) delta_groups_kernel(const DgArgs a) {
+  pdl_wait(); pdl_trigger();
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  const int lane = threadIdx.x & 31;
+  // Of the sequences that are long enough the blockIdx.y-th, and every gridDim.y-th behind it.  Up to 64 in the order of their lengths, longest first: lanes hold a
+  // number that grows with the length and tells equal ones apart, for two sequences each.  More as they come (so many fill the SMs several times over, and the
+  // last wave weighs less), without counting where there is a CTA for each.
+  auto length = [&](int s) { return s < a.B ? a.cu[s + 1] - a.cu[s] : 0; };
+  auto fit = [&](int n) { return n >= a.min_n && n < a.max_n; };
+  unsigned key[2] = {0, 0};
+  if (a.B <= 64)
+#pragma unroll
+    for (int i = 0; i < 2; i++) { const int s = lane + 32 * i, n = length(s); if (fit(n)) key[i] = (unsigned)min(n, 1 << 25) << 6 | (63 - s); }
+  int at = 0, from = 0, before = 0;            // as they come: sequences in front of `from` hold `before` that fit
+  for (int y = blockIdx.y; ; y += gridDim.y) {
+    int seq = -1;
+    if (a.B <= 64) {
+      unsigned top = 0;
+      for (; at <= y; at++) {
+        top = __reduce_max_sync(0xffffffffu, max(key[0], key[1]));
+        if (key[0] == top) key[0] = 0;
+        if (key[1] == top) key[1] = 0;
+      }
+      if (top) seq = 63 - (int)(top & 63);
+    } else if ((int)gridDim.y == a.B) {
+      if (y < a.B && fit(length(y))) seq = y;
+    } else {
+      for (; from < a.B; from += 32) {
+        const unsigned all = __ballot_sync(0xffffffffu, fit(length(from + lane)));
+        if (y < before + __popc(all)) {
+          seq = from + __ffs(__ballot_sync(0xffffffffu, (all >> lane & 1) && before + __popc(all & ((1u << lane) - 1)) == y)) - 1;
+          break;
+        }
+        before += __popc(all);
+      }
+    }
+    if (seq < 0) return;
+    if (y != (int)blockIdx.y) __syncthreads();          // shared memory is the next one's
+    delta_groups_sequence<kVec>(a, seq, smem_raw);
+  }
+}
+
 }  // namespace ne
 
 using namespace ne;
 
-// Sequences of less than max_n tokens in this call (the others are left alone).  q, k [T, Hk, 128] (row stride qk_ld), v [T, H, 128] (v_ld), b [T, >= H] (b_ld);
-// per_channel: g [T, H, 128] contiguous, dt_bias [H, 128], log decays lower_bound sigmoid(e^A (g + bias)) if lower_bound < 0, else -e^A softplus(g + bias);
-// otherwise g [T, >= H] (g_ld), dt_bias [H], -e^A softplus.  Rows of q, k, v, per-channel g and the state on 16-byte boundaries.  raw fp32 [T, H, 128].
-extern "C" int ne_delta_groups(const void* q, const void* k, const void* v, const void* g, const void* b, long long qk_ld, long long v_ld, long long g_ld,
-                               long long b_ld, const float* A_log, const float* dt_bias, float lower_bound, float* state, const int* slots, const int* cu,
-                               const int* fresh, float* raw, int B, int Hk, int H, int max_n, int per_channel, cudaStream_t st) {
+static int dg_sms() {
+  static int n = 0;
+  if (!n) { int dev; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); }
+  return n;
+}
+
+extern "C" int ne_gdn_step(const void* q, const void* k, const void* v, long long qk_ld, long long v_ld, const void* a, const void* b, long long ab_ld,
+                           const float* A_log, const float* dt_bias, float* state, const int* slots, const int* cu, const int* fresh, const void* z,
+                           long long z_ld, const void* norm_w, float eps, void* out, long long out_ld, int B, int Hk, int Hv, int Dk, int Dv, int skip_len,
+                           int raw_out, int vec_gate, float lower_bound, cudaStream_t st);
+
+// Sequences of less than max_n tokens in this call (the others are left alone): those of at least min_n (> 0) four tokens at a time, if `groups`, those of less
+// token by token, if `step`, so that which form a sequence takes is its own length's matter and not its neighbours'.  q, k [T, Hk, 128] (row stride qk_ld),
+// v [T, H, 128] (v_ld), b [T, >= H] (b_ld); per_channel: g [T, H, 128] contiguous, dt_bias [H, 128], log decays lower_bound sigmoid(e^A (g + bias)) if
+// lower_bound < 0, else -e^A softplus(g + bias); otherwise g [T, >= H] (rows as b's), dt_bias [H], -e^A softplus.  Rows of q, k, v, per-channel g and the state on
+// 16-byte boundaries.  raw fp32 [T, H, 128].
+extern "C" int ne_delta_portions(const void* q, const void* k, const void* v, const void* g, const void* b, long long qk_ld, long long v_ld, long long b_ld,
+                                 const float* A_log, const float* dt_bias, float lower_bound, float* state, const int* slots, const int* cu, const int* fresh,
+                                 float* raw, int T, int B, int Hk, int H, int min_n, int max_n, int step, int groups, int per_channel, cudaStream_t st) {
   if (B <= 0) return 0;
-  if (Hk < 1 || H % Hk || B > 65535) return 1001;
+  if (Hk < 1 || H % Hk || B > 65535 || min_n < 1) return 1001;
   if (qk_ld % 8 || v_ld % 8 || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)state) & 15) || (per_channel && ((uintptr_t)g & 15))) return 1002;
+  if (step) {
+    const int rc = ne_gdn_step(q, k, v, qk_ld, v_ld, g, b, b_ld, A_log, dt_bias, state, slots, cu, fresh, nullptr, 0, nullptr, 0.f, raw, (long long)H * 128, B, Hk, H,
+                               128, 128, min(min_n, max_n), 1, per_channel, lower_bound, st);
+    if (rc) return rc;
+  }
+  // No more than T / min_n can be long enough.  Where most sequences are shorter, a wave of CTAs, which then take several, costs less than one for each that may
+  // find nothing to do: 64 portions of 2 tokens, 32 heads: 70 us against 77, without this kernel 68.
+  const int rows = T >= min_n * B ? B : min(T / min_n, (3 * dg_sms() + 2 * H - 1) / (2 * H));
+  if (!groups || rows < 1) return 0;
   DgArgs a;
   a.q = (const __nv_bfloat16*)q; a.k = (const __nv_bfloat16*)k; a.v = (const __nv_bfloat16*)v; a.g = (const __nv_bfloat16*)g; a.b = (const __nv_bfloat16*)b;
-  a.qk_ld = qk_ld; a.v_ld = v_ld; a.g_ld = g_ld; a.b_ld = b_ld; a.A_log = A_log; a.dt_bias = dt_bias; a.lower_bound = lower_bound; a.state = state;
-  a.slots = slots; a.cu = cu; a.fresh = fresh; a.raw = raw; a.B = B; a.H = H; a.rep = H / Hk; a.max_n = max_n;
+  a.qk_ld = qk_ld; a.v_ld = v_ld; a.g_ld = b_ld; a.b_ld = b_ld; a.A_log = A_log; a.dt_bias = dt_bias; a.lower_bound = lower_bound; a.state = state;
+  a.slots = slots; a.cu = cu; a.fresh = fresh; a.raw = raw; a.B = B; a.H = H; a.rep = H / Hk; a.min_n = min_n; a.max_n = max_n;
   auto kern = per_channel ? delta_groups_kernel<true> : delta_groups_kernel<false>;
   static bool configured[2] = {false, false};
   if (!configured[per_channel != 0]) {
@@ -323,5 +373,5 @@ extern "C" int ne_delta_groups(const void* q, const void* k, const void* v, cons
     if (e != cudaSuccess) return (int)e;
     configured[per_channel != 0] = true;
   }
-  return (int)launch_pdl(kern, dim3((unsigned)(2 * H), (unsigned)B), dim3(kDgThreads), kDgSmem, st, a);
+  return (int)launch_pdl(kern, dim3((unsigned)(2 * H), (unsigned)rows), dim3(kDgThreads), kDgSmem, st, a);
 }

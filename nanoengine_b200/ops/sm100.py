@@ -1103,23 +1103,27 @@ def rmsnorm_gated(x: torch.Tensor, z: torch.Tensor, w: torch.Tensor, eps: float,
     return out
 
 
-def _delta_groups(q, k, v, g, b, A_log, dt_bias, lower_bound, state, slots, cu, fresh, raw, max_n, per_channel):
-    """Four tokens at a time, 128 x 128 states, the sequences of less than `max_n` new tokens."""
-    _ck(lib().ne_delta_groups(_p(q), _p(k), _p(v), _p(g), _p(b), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _c.c_longlong(g.stride(0)),
-                              _c.c_longlong(b.stride(0)), _p(A_log), _p(dt_bias), _c.c_float(lower_bound), _p(state), _p(slots), _p(cu), _p(fresh), _p(raw),
-                              _c.c_int(cu.numel() - 1), _c.c_int(q.shape[1]), _c.c_int(v.shape[1]), _c.c_int(max_n), _c.c_int(1 if per_channel else 0), _st()),
-        "ne_delta_groups")
-
-
 def _delta_rows16(q, k, v, state):
     """128 x 128 states with rows that the prompt kernels of the delta rule can copy in 16-byte pieces."""
     return (q.shape[2] == v.shape[2] == 128 and q.stride(0) % 8 == 0 and k.stride(0) == q.stride(0) and v.stride(0) % 8 == 0
             and all(t.data_ptr() % 16 == 0 for t in (q, k, v, state)))
 
 
-# Mean portion (tokens) above which four tokens at a time beat one at a time: us for one / four, 32 heads: 64 portions of 2: 72 / 92, 4 of 8: 52 / 53 (both
-# the host's), 16 of 16: 106 / 53, 11 of 55 (16 heads): 153 / 66, 16 of 370: 2208 / 724
-GROUPS_MIN_MEAN = 4
+# Portion (tokens) from which four tokens at a time beat one at a time: us for one / four, 32 heads: 64 portions of 2: 72 / 92, 4 of 8: 52 / 53 (both the
+# host's), 16 of 16: 106 / 53, 11 of 55 (16 heads): 153 / 66, 16 of 370: 2208 / 724.  By its own length, whatever the batch: a prompt beside decode steps
+# does not take their form (and sums in the same order as alone), nor they its.
+GROUPS_MIN = 5
+
+
+def _delta_portions(q, k, v, g, b, A_log, dt_bias, lower_bound, state, slots, cu, fresh, raw, max_n, per_channel, lens=None):
+    """128 x 128 states, the sequences of less than `max_n` new tokens: four tokens at a time from GROUPS_MIN on, one at a time below.  `lens`: lengths of all that are
+    not empty (and not longer), where the host knows them."""
+    step, groups = (True, True) if lens is None else (min(lens) < GROUPS_MIN, max(lens) >= GROUPS_MIN)
+    _ck(lib().ne_delta_portions(_p(q), _p(k), _p(v), _p(g), _p(b), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _c.c_longlong(b.stride(0)), _p(A_log),
+                                _p(dt_bias), _c.c_float(lower_bound), _p(state), _p(slots), _p(cu), _p(fresh), _p(raw), _c.c_int(q.shape[0]), _c.c_int(cu.numel() - 1),
+                                _c.c_int(q.shape[1]), _c.c_int(v.shape[1]), _c.c_int(GROUPS_MIN), _c.c_int(max_n), _c.c_int(int(step)), _c.c_int(int(groups)),
+                                _c.c_int(1 if per_channel else 0), _st()), "ne_delta_portions")
+    LAUNCHES[0] += step and groups
 
 
 def _gdn_step(q, k, v, a, b, A_log, dt_bias, state, slots, cu, fresh, z, norm_w, eps, dst, skip, raw):
@@ -1158,11 +1162,9 @@ def gdn_recurrent(q, k, v, a, b, A_log, dt_bias, state, slots, cu_seqlens, fresh
             _ck(lib().ne_delta_chunk(_p(q), _p(k), _p(v), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _p(a), _p(b), _c.c_longlong(a.stride(0)),
                                      _p(A_log), _p(dt_bias), _p(state), _p(slots), _p(cu), _p(fresh), _p(raw), _p(work), _c.c_int(T), _c.c_int(cu.numel() - 1),
                                      _c.c_int(chunks), _c.c_int(Hk), _c.c_int(Hv), _c.c_int(skip), _st()), "ne_delta_chunk")
-            short = [e - s for s, e in zip(cu_host, cu_host[1:]) if e - s < skip]
-            if sum(short) > GROUPS_MIN_MEAN * len(short):
-                _delta_groups(q, k, v, a, b, A_log, dt_bias, 0.0, state, slots, cu, fresh, raw, skip, False)
-            elif short:
-                _gdn_step(q, k, v, a, b, A_log, dt_bias, state, slots, cu, fresh, z, norm_w, eps, raw, skip, True)
+            short = [e - s for s, e in zip(cu_host, cu_host[1:]) if s < e < s + skip]
+            if short:
+                _delta_portions(q, k, v, a, b, A_log, dt_bias, 0.0, state, slots, cu, fresh, raw, skip, False, short)
             return rmsnorm_gated(raw, z, norm_w, eps, out).view(T, Hv * Dv)
         rep = Hv // Hk
         g, beta = ref.gdn_gates(a, b, A_log, dt_bias)
@@ -1177,9 +1179,9 @@ def gdn_recurrent(q, k, v, a, b, A_log, dt_bias, state, slots, cu_seqlens, fresh
             o, S = ref.gdn_chunked(qn, kn, v[s:e].float(), g[s:e], beta[s:e], S0)
             state.index_copy_(0, sl, S[None])
             rmsnorm_gated(o, z[s:e], norm_w, eps, out[s:e])
-    elif T > GROUPS_MIN_MEAN * (cu.numel() - 1) and _delta_rows16(q, k, v, state):
+    elif (max_q_len >= GROUPS_MIN or T >= GROUPS_MIN * (cu.numel() - 1)) and _delta_rows16(q, k, v, state):
         raw = torch.empty(T, Hv, Dv, dtype=torch.float32, device=q.device)
-        _delta_groups(q, k, v, a, b, A_log, dt_bias, 0.0, state, slots, cu, fresh, raw, skip, False)
+        _delta_portions(q, k, v, a, b, A_log, dt_bias, 0.0, state, slots, cu, fresh, raw, skip, False, None if cu_host is None or T == 0 else [e - s for s, e in zip(cu_host, cu_host[1:]) if s < e] or None)
         return rmsnorm_gated(raw, z, norm_w, eps, out).view(T, Hv * Dv)
     raw = bool(lib().ne_gdn_step_raw_only(_c.c_int(Dk), _c.c_int(Dv)))     # large states: several CTAs per head, norm in its own kernel
     if raw and max_q_len >= ref.GDN_CHUNK_MIN_TOKENS:
@@ -1337,8 +1339,8 @@ def kda_recurrent(q, k, v, raw_g, b, A_log, dt_bias, lower_bound, state, slots, 
     slots, cu, fresh = _i32(slots), _i32(cu_seqlens), _i32(fresh)
     raw = torch.empty(T, H, Dv, dtype=torch.float32, device=q.device)
     lb = float(lower_bound) if lower_bound is not None else 0.0
-    if T > GROUPS_MIN_MEAN * (cu.numel() - 1) and _delta_rows16(q, k, v, state) and raw_g.data_ptr() % 16 == 0:
-        _delta_groups(q, k, v, raw_g, b, A_log, dt_bias, lb, state, slots, cu, fresh, raw, 1 << 30, True)
+    if T > cu.numel() - 1 and _delta_rows16(q, k, v, state) and raw_g.data_ptr() % 16 == 0:
+        _delta_portions(q, k, v, raw_g, b, A_log, dt_bias, lb, state, slots, cu, fresh, raw, 1 << 30, True)
     else:
         _ck(lib().ne_gdn_step(_p(q), _p(k), _p(v), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _p(raw_g), _p(b), _c.c_longlong(b.stride(0)),
                               _p(A_log), _p(dt_bias), _p(state), _p(slots), _p(cu), _p(fresh), _p(gate), _c.c_longlong(gate.stride(0)), _p(norm_w),

@@ -174,3 +174,31 @@ def test_strided_gates_and_tables(lens):
                                1e-6, max(lens), cu)
     got = sm100.gdn_recurrent(q, k, v, ab[..., 0], ab[..., 1], A[:, 1], bias[:, 2], two, table[:, 0], ends[:, 0], table[:, 1], z, w2[:, 0], 1e-6, max(lens), cu)
     assert torch.equal(got, want) and torch.equal(one, two)
+
+
+@pytest.mark.parametrize("per_channel", [False, True])
+@pytest.mark.parametrize("n", [2, 4, 5, 30, 64, 130])
+@pytest.mark.parametrize("others", [[1] * 40, [1] * 30 + [7] * 50, [100, 1]])
+def test_a_sequence_does_not_depend_on_its_batch(per_channel, n, others):
+    """Bit for bit: which form the rule takes, and in which order it sums, is a matter of the sequence's own length."""
+    from nanoengine_b200.ops import sm100
+    hk, hv, at = (2, 2, len(others) // 2) if per_channel else (2, 4, len(others) // 2)
+    lens = others[:at] + [n] + others[at:]
+    gen, r, q, k, v, state, slots, fresh, cu, z, w = _inputs(lens, hk, hv, 13)
+    t, fresh = sum(lens), torch.zeros_like(fresh)
+    a, b = r(t, hv * (D if per_channel else 1)).to(torch.bfloat16), r(t, hv).to(torch.bfloat16)
+    A, bias = torch.zeros(hv, device="cuda"), torch.zeros(hv * (D if per_channel else 1), device="cuda")
+
+    def run(rows, lens, st, sl, fr, host):
+        ends = [0] + torch.tensor(lens).cumsum(0).tolist()
+        x, c = [i[rows] for i in (q, k, v, a, b)], torch.tensor(ends, dtype=torch.int32, device="cuda")
+        if per_channel:
+            return sm100.kda_recurrent(*x, A, bias, -5.0, st, sl, c, fr, z[rows], w, 1e-6)
+        return sm100.gdn_recurrent(*x, A, bias, st, sl, c, fr, z[rows], w, 1e-6, max(lens), ends if host or max(lens) >= 64 else None)
+
+    for host in (False, True):
+        one, all_ = state.clone(), state.clone()
+        own = slice(cu[at], cu[at + 1])
+        alone = run(own, [n], one, slots[at: at + 1], fresh[at: at + 1], host)
+        batch = run(slice(0, t), lens, all_, slots, fresh, host)
+        assert torch.equal(batch[own], alone) and torch.equal(all_[slots[at].long()], one[slots[at].long()])
