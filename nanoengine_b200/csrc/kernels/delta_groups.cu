@@ -18,6 +18,7 @@
 
 namespace ne {
 
+[[maybe_unused]] constexpr int kKernelDg = 29;      // in status words of the checked build
 constexpr int kDgTok = 16;                     // tokens per stage
 constexpr int kDgRows = 64;                    // state rows per CTA
 constexpr int kDgThreads = 128;
@@ -65,7 +66,7 @@ __device__ __forceinline__ void delta_groups_sequence(const DgArgs& a, int seq, 
   const int h = blockIdx.x >> 1, row0 = (blockIdx.x & 1) * kDgRows, hk = h / a.rep;
   const int start = a.cu[seq], n = a.cu[seq + 1] - start;
   const int slot = a.slots[seq];
-  if (!NE_INDEX_OK(slot, BK_STATE_SLOTS, 28, __LINE__)) return;
+  if (!NE_INDEX_OK(slot, BK_STATE_SLOTS, kKernelDg, __LINE__)) return;
   // lane: rows row0 + warp 16 + r 4 + grp, columns i 32 + sub 4 ..
   float* Sg = a.state + (((long long)slot * a.H + h) * 128 + row0 + warp * 16 + grp) * 128 + sub * 4;
   f32x2 S[4][8];

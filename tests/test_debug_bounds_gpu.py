@@ -74,3 +74,34 @@ def test_checked_build_catches_bad_entries_and_runs_the_engine():
     checked = _run({"NE_DEBUG_BOUNDS": "1"})
     plain = _run({"NE_DEBUG_BOUNDS": "0"})
     assert checked == plain
+
+
+_SLOTS = r"""
+import torch
+from nanoengine_b200.ops import sm100
+assert sm100.lib()._name.endswith("libne_kernels_dbg.so")
+assert sm100.debug_set_bounds(cache_rows=0, cache_pages=0, state_slots=2, experts=0)      # of the four that are allocated
+seen = []
+for n, kernels in ((2, 21), (9, 29), (70, 28)):         # one token at a time, four, a chunk
+    sm100.clear_kernel_status()
+    y = torch.randn(n, 3, 128, device="cuda", dtype=torch.bfloat16)
+    q, k, v = y[:, :1], y[:, 1:2], y[:, 2:]
+    a = torch.zeros(n, 1, device="cuda", dtype=torch.bfloat16)
+    state = torch.ones(4, 1, 128, 128, device="cuda")
+    one = lambda *x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    sm100.gdn_recurrent(q, k, v, a, a, torch.zeros(1, device="cuda"), torch.zeros(1, device="cuda"), state, one(3), one(0, n), one(0), v, torch.ones(128, device="cuda", dtype=torch.bfloat16),
+                        1e-6, n, [0, n])
+    torch.cuda.synchronize()
+    st = sm100.kernel_status()
+    assert st[0] == 4 and st[1] == kernels and st[4] == 3, (n, st)                          # which kernel met the bad slot
+    assert (state == 1).all()
+print("TOKENS")
+"""
+
+
+def test_checked_build_names_the_delta_rule_kernel_that_met_a_bad_slot():
+    from nanoengine_b200.build_native import build_kernels
+    build_kernels(debug_bounds=True)
+    r = subprocess.run([sys.executable, "-c", _SLOTS], env=dict(os.environ, NE_DEBUG_BOUNDS="1"), capture_output=True, text=True, timeout=280,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-3000:]
