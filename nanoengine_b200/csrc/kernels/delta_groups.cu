@@ -300,18 +300,19 @@ __global__ void __launch_bounds__(kDgThreads, 3) delta_groups_kernel(const DgArg
 #pragma unroll
     for (int i = 0; i < 2; i++) { const int s = lane + 32 * i, n = length(s); if (fit(n)) key[i] = (unsigned)min(n, 1 << 25) << 6 | (63 - s); }
   int at = 0, from = 0, before = 0;            // as they come: sequences in front of `from` hold `before` that fit
-  for (int y = blockIdx.y; ; y += gridDim.y) {
+  for (int y = blockIdx.y; y < a.B; y += gridDim.y) {
     int seq = -1;
     if (a.B <= 64) {
       unsigned top = 0;
       for (; at <= y; at++) {
         top = __reduce_max_sync(0xffffffffu, max(key[0], key[1]));
+        if (!top) return;
         if (key[0] == top) key[0] = 0;
         if (key[1] == top) key[1] = 0;
       }
-      if (top) seq = 63 - (int)(top & 63);
+      seq = 63 - (int)(top & 63);
     } else if ((int)gridDim.y == a.B) {
-      if (y < a.B && fit(length(y))) seq = y;
+      if (fit(length(y))) seq = y;
     } else {
       for (; from < a.B; from += 32) {
         const unsigned all = __ballot_sync(0xffffffffu, fit(length(from + lane)));

@@ -1115,14 +1115,26 @@ def _delta_rows16(q, k, v, state):
 GROUPS_MIN = 5
 
 
+_PORTIONS = []
+
+
+def _portions_call():
+    """The entry with declared arguments: plain integers cost a fraction of wrapped ones, and small batches are the host's time."""
+    if not _PORTIONS:
+        f, i, p, n, x = lib().ne_delta_portions, _c.c_int, _c.c_void_p, _c.c_longlong, _c.c_float
+        f.argtypes = [p, p, p, p, p, n, n, n, p, p, x, p, p, p, p, p, i, i, i, i, i, i, i, i, i, p]
+        _PORTIONS.append(f)
+    return _PORTIONS[0]
+
+
 def _delta_portions(q, k, v, g, b, A_log, dt_bias, lower_bound, state, slots, cu, fresh, raw, max_n, per_channel, lens=None):
     """128 x 128 states, the sequences of less than `max_n` new tokens: four tokens at a time from GROUPS_MIN on, one at a time below.  `lens`: lengths of all that are
     not empty (and not longer), where the host knows them."""
     step, groups = (True, True) if lens is None else (min(lens) < GROUPS_MIN, max(lens) >= GROUPS_MIN)
-    _ck(lib().ne_delta_portions(_p(q), _p(k), _p(v), _p(g), _p(b), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _c.c_longlong(b.stride(0)), _p(A_log),
-                                _p(dt_bias), _c.c_float(lower_bound), _p(state), _p(slots), _p(cu), _p(fresh), _p(raw), _c.c_int(q.shape[0]), _c.c_int(cu.numel() - 1),
-                                _c.c_int(q.shape[1]), _c.c_int(v.shape[1]), _c.c_int(GROUPS_MIN), _c.c_int(max_n), _c.c_int(int(step)), _c.c_int(int(groups)),
-                                _c.c_int(1 if per_channel else 0), _st()), "ne_delta_portions")
+    _ck(_portions_call()(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), b.data_ptr(), q.stride(0), v.stride(0), b.stride(0), A_log.data_ptr(),
+                         dt_bias.data_ptr(), lower_bound, state.data_ptr(), slots.data_ptr(), cu.data_ptr(), fresh.data_ptr(), raw.data_ptr(), q.shape[0],
+                         cu.numel() - 1, q.shape[1], v.shape[1], GROUPS_MIN, max_n, step, groups, per_channel, torch.cuda.current_stream().cuda_stream),
+        "ne_delta_portions")
     LAUNCHES[0] += step and groups
 
 
