@@ -18,9 +18,9 @@
 // Sums of log decays are 64-bit (64 numbers a chunk): a factor between two tokens is the exponential of a difference of sums.  The tensor cores cut off
 // what falls below an accumulator's last bit, so the state is not an accumulator of theirs: a chunk's products are summed from zero and then added.
 //
-// Bound: the matrix instructions of the scan (190 a chunk and warp, 8 cycles each on a scheduler: 3,000 cycles for 64 tokens x 32 columns, beside as many of
-// shared memory), and its chain of products.  Measured: 4 prompts of 750 .. 2250 tokens, 32 heads over 16: 14774 us as batched fp32 products and triangular
-// solves of a library per sequence, 571 us so.  Errors against 64 bits: final states 1.8e-7 (before: 1.8e-7), outputs in front of the norm 4.3e-7 (3.6e-6 with two
+// Bound: the scan's chain of four products a chunk, two CTAs per SM: tensor pipe 49 % busy, shared memory and barriers between the products the rest; in the
+// preparation the barriers between its steps (issue slots 51 % busy).  Measured: 4 prompts of 750 .. 2250 tokens, 32 heads over 16: 14774 us as batched fp32 products and triangular
+// solves of a library per sequence, 571 us so (under a profiler: prepare 172, scan 371, norm 55).  Errors against 64 bits: final states 1.8e-7 (before: 1.8e-7), outputs in front of the norm 4.3e-7 (3.6e-6 with two
 // terms of P T and of R).
 //
 // Replaces in the reference: the chunked prefill of triton/fla (layers/backends/delta_net/components/recurrence.py:100-200).

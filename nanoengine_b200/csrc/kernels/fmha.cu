@@ -9,8 +9,8 @@
 //     P(j) = exp2(S - m)  one warpgroup per tile; bf16 pairs written over S(j) in TMEM, the A operand of the second product
 //     O   += P(j) V       (N = head size up to the next multiple of 16; V read MN-major)
 // The softmax finds S(j+1) ready when it has handed P(j) on.  (Blocks of 128 keys with one slot a tile read less shared memory per product, but then scores,
-// softmax and products of a tile are one chain: 4150 cycles for 128 keys of two tiles, whether one or two warpgroups share a tile's softmax; so it is 4000.  One
-// tile per CTA and two CTAs per SM, or an issuer each for scores and products, were no faster.)
+// softmax and products of a tile are one chain, whether one or two warpgroups share a tile's softmax: slower.  One tile per CTA and two CTAs per SM, or an issuer
+// each for scores and products, were slower for long prompts too.)
 // The order of two products is promised only where they share accumulator and shape, so S(j+2) waits for the products that read the slot: PV(j) itself with two
 // slots, which the other tile's products, or the other CTA's, fill (1063 -> 1088 us for the MLA prompts below, against issuing without the wait), PV(j-1) with
 // three (256-wide heads, nothing beside them: 177 without a wait, 197 with two slots, 186 so).
@@ -24,11 +24,11 @@
 // memory before their product: 0 x inf there would reach the result.  Values that some rows of a tile see and others do not: fmha_row_again.  Warp 0: TMA producer, 1 and 2: MMA issuers of tile 0 and 1, 3: that zeroing,
 // 4-7 / 8-11: softmax, rescale and epilogue of tile 0 / 1.  All waits are bounded.
 //
-// Bound: products issued on their own (no softmax) take 75 - 85 % of the time; 64 keys of two tiles take 1960 cycles, of which the tensor pipe could do with
-// 1280 (operand reads of N = 64) and the exponentials with 1024.  Measured (B200, us, before -> so): 64 / 4 heads of 128, prompts of 1024 .. 3072 tokens, 8192
-// in all: 574 -> 423 (gqa_bf16.cu, one tile, one CTA per SM); MLA, 128 heads, the same prompts: 1323 -> 1089 (that kernel); 16 / 4 heads of 256, window 1024,
-// 6000 tokens: 51740 -> 162 and 16 heads of 72, 5 images of 600 .. 1800 patches: 143260 -> 111 (attn_generic.cu, a token and four heads per CTA on the CUDA
-// cores).
+// Bound: the hand-overs between scores, softmax and products; no unit is full (busy % of the tensor pipe / exponentials / issue slots: MLA prompts 42 / 34 / 39,
+// GQA 37 / 38 / 39, windows of 256-wide heads 43 / 15 / 24, vision 34 / 38 / 45).  Measured (B200, us, before -> so): 64 / 4 heads of 128, prompts of 1024 .. 3072
+// tokens, 8192 in all: 574 -> 415 (gqa_bf16.cu, one tile, one CTA per SM); MLA, 128 heads, the same prompts: 1323 -> 1080 (that kernel); 16 / 4 heads of 256,
+// window 1024, 6000 tokens: 51740 -> 157 and 16 heads of 72, 5 images of 600 .. 1800 patches: 143260 -> 116 (attn_generic.cu, a token and four heads per CTA on the
+// CUDA cores).
 //
 // Replaces in the reference: the FA4 / FA3 varlen prefill calls (layers/backends/attention/fa4.py:34-245, fa3.py), the ragged MLA prefill of
 // models/deepseek_v2/deepseek_v2.py:1792-1816, and the varlen attention of the vision encoder.

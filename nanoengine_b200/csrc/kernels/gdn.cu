@@ -1,10 +1,11 @@
 // Gated delta-net linear attention (Qwen3.5 family): the memory-bound pieces.
 //   * causal depthwise convolution + SiLU over ragged sequences with a carried window of the last K-1 inputs per sequence
-//   * the recurrent delta rule: one CTA per (sequence, value head) keeps the whole [Dv, Dk] fp32 state in registers, walks the
+//   * the recurrent delta rule, token by token: CTAs of a (sequence, value head) keep its [Dv, Dk] fp32 state in registers, walk the
 //     sequence's new tokens, and applies the gated RMSNorm to each output row before it leaves the SM.  A decode step reads
 //     and writes the state exactly once (the op's floor: 2 * Dv * Dk * 4 bytes per head), everything else is a few KB.
 //   * gated RMSNorm alone, for outputs produced by the chunked (matrix-product) prefill form
-// Long prefill sequences run the chunked form on batched matrix products; this kernel serves decode, verification and short chunks.
+// It serves decode, verification and portions of less than five tokens; longer ones of 128 x 128 states run in delta_groups.cu and delta_chunk.cu, long ones of
+// other sizes as batched matrix products.
 // Replaces in the reference: layers/backends/delta_net/components/conv.py (causal_conv1d calls and the naive conv),
 // components/recurrence.py:100-200, components/output.py:17-62, triton/fla/fused_recurrent.py, triton/generic/rmsnorm_gated.py.
 #include "ptx.cuh"
@@ -266,7 +267,8 @@ __global__ void __launch_bounds__(256) rmsnorm_gated_kernel(const float* __restr
 }
 
 // The same for D = 128 and rows on 8-byte boundaries: four neighbouring columns a lane, kRows rows a warp whose loads are all under way before the first is
-// used.  Bound by memory (8 bytes a column); 192,000 rows: 71 us with 2-byte accesses and one row a warp, 53 us so (3.7 TB/s).
+// used.  192,000 rows: 71 us with 2-byte accesses and one row a warp, 53 us so (3.7 TB/s for 8 bytes a column, DRAM 40 % busy), bound by the unit of the
+// exponentials and reciprocals of the gate (74 % busy).
 constexpr int kNormRows = 4;
 __global__ void __launch_bounds__(256) rmsnorm_gated128_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ z, long long z_ld,
                                                               const __nv_bfloat16* __restrict__ w, float eps, __nv_bfloat16* __restrict__ out,

@@ -900,7 +900,7 @@ def attention_varlen(q, k, v, cu_seqlens, scale, causal: bool = False):
 
 
 def mla_prefill_ragged(q: torch.Tensor, k_nope: torch.Tensor, k_rope: torch.Tensor, v: torch.Tensor, cu_seqlens, scale: float) -> torch.Tensor:
-    """Non-absorbed MLA prefill attention on the tcgen05 prompt kernel (pairs of 128-query tiles per head, 128-key blocks fetched by token
+    """Non-absorbed MLA prefill attention on the tcgen05 prompt kernel (pairs of 128-query tiles per head, 64-key blocks fetched by token
     coordinate, the shared rotary key part through its own tensor map): head dims 128 + 64 / 128 only."""
     T, H, D = q.shape
     assert D == 192 and k_nope.shape == (T, H, 128) and v.shape == (T, H, 128) and k_rope.shape == (T, 64)

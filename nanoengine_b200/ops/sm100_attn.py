@@ -181,6 +181,11 @@ def _fmha_covers(group: int, D: int, Dv: int) -> bool:
     return 1 <= group <= 128 and 8 <= D <= 256 and D % 8 == 0 and 8 <= Dv <= 256 and Dv % 8 == 0
 
 
+# Key slices at most: each writes an fp32 partial result that the merge reads again.  us at 16 / 32 / 64: four decode tokens over 16K keys, two KV heads of 256:
+# 39.6 / 42.9 / 42.9; one token: 35.5 / 28.8 / 31.8, over 64K keys 105 / 64 / 51, over 4K 18.3 whatever the limit (one or two long contexts would gain from more)
+FMHA_MAX_SLICES = 16
+
+
 def _fmha_tiles(T: int, B: int, Hq: int, Hkv: int, D: int, Dv: int) -> int:
     """Tiles of 128 rows per CTA.  Two share the keys they read; TMEM holds two accumulators of up to 128 columns, shared memory two Q tiles of up to 192.  One
     where single ones fit a wave or a portion is less than one; us for one / two (MLA): a prompt of 2000, 16 heads: 68 / 48; 8 of 64, 128 heads: 40 / 57"""
@@ -198,9 +203,9 @@ def _fmha(q, k, v, cu, scale, causal, split_p, block_tables=None, context_lens=N
     rows = tq * tiles
     grid = min(T, T // rows + B)
     S = 1
-    if paged and grid * Hkv < _sms() // 2:             # few CTAs (small decode batches, short prompts): slice the keys, blocks of 128
+    if paged and grid * Hkv < _sms() // 2:             # few CTAs (small decode batches, short prompts): slice the keys, at least four pages of 64 each
         pages = block_tables.shape[1] if window <= 0 else min(block_tables.shape[1], (window + rows + 126) // 64 + 1)
-        S = max(1, min(_sms() // (grid * Hkv), max(1, pages // 4), 16))
+        S = max(1, min(_sms() // (grid * Hkv), max(1, pages // 4), FMHA_MAX_SLICES))
     out = torch.empty(T, Hq, Dv, dtype=torch.bfloat16, device=q.device)
     part = lse2 = None
     if S > 1:
@@ -239,7 +244,8 @@ def gqa_attention_paged(q, k_cache, v_cache, block_tables, cu_seqlens_q, context
                and k_cache.is_contiguous() and v_cache.is_contiguous())
     if D == 128 and window <= 0 and pages64 and group & (group - 1) == 0:
         q = q.contiguous()
-        # The prompt kernel where its tiles fill the SMs and the portions fill tiles; else the kernel of the decode steps, whose results are the same.  us for that /
+        # The prompt kernel where its tiles fill the SMs and the portions fill tiles; else the kernel of the decode steps, which rounds the same probabilities and sums
+        # them in another order (a value is at most one step of bf16 apart, fewer than one in a hundred are).  us for that /
         # this, 64 / 4 heads: 4 prompts of 1000: 183 / 138, one of 600 (304 tiles): 26 / 20; 8 / 1 heads, one of 2000 (126 tiles): 31 / 38; 128 x 2 tokens: 150 / 172
         tq = 128 // group
         if T >= B * tq and min(T, T // tq + B) * Hkv > _sms():

@@ -58,7 +58,7 @@ def test_paged(hq, hkv, dim, window, new, total):
     calls = sm100_attn.PROMPT_TC_CALLS[0]
     tq, t = 128 // (hq // hkv), sum(new)
     plain = dim == 128 and window == 0
-    prompt = not plain or (t >= len(new) * tq and min(t, t // tq + len(new)) * hkv > 148)
+    prompt = not plain or (t >= len(new) * tq and min(t, t // tq + len(new)) * hkv > sm100_attn._sms())
     if not prompt:
         vc, kc = vc.nan_to_num(0.0), kc.nan_to_num(0.0)    # the decode kernel multiplies whole pages
     got = sm100_attn.gqa_attention_paged(q, kc, vc, bt, cu, torch.tensor(total, dtype=torch.int32, device="cuda"), dim ** -0.5, window)
@@ -232,3 +232,23 @@ def test_boundaries_past_the_tensors_end_write_nothing_there():
     for cu in (torch.tensor([0, t], dtype=torch.int32), torch.tensor([0], dtype=torch.int32, device="cuda")):
         with pytest.raises(AssertionError):
             sm100.attention_varlen(q[:t], k[:t], v[:t], cu, 0.1)
+
+
+def test_a_prompt_alone_and_in_a_batch():
+    """Alone its tiles do not fill the SMs and the decode steps' kernel takes it, in a batch the prompt kernel does.  Both round the same probabilities to bf16 and sum
+    them in 32 bits, in another order: a few 2^-24 apart before the results are rounded to bf16, so some of them one step (2^-7 of a value at most) apart, few."""
+    from nanoengine_b200.ops import sm100_attn
+    g = torch.Generator(device="cuda").manual_seed(14)
+    n, hq, hkv = sm100_attn._sms() * 8 // 6, 64, 4             # 8 tokens a tile: two thirds of a wave, twice that in the batch
+    nb = -(-n // 64)
+    kc, vc = (torch.randn(2 * nb, 64, hkv, 128, generator=g, device="cuda").to(torch.bfloat16) for _ in "kv")
+    q = torch.randn(2 * n, hq, 128, generator=g, device="cuda").to(torch.bfloat16)
+    bt = torch.arange(2 * nb, dtype=torch.int32, device="cuda").view(2, nb)
+    cu, cl = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([0, n, 2 * n], [n, n]))
+    calls = sm100_attn.PROMPT_TC_CALLS[0]
+    alone = sm100_attn.gqa_attention_paged(q[:n], kc, vc, bt[:1], cu[:2], cl[:1], 128 ** -0.5)
+    assert sm100_attn.PROMPT_TC_CALLS[0] == calls
+    both = sm100_attn.gqa_attention_paged(q, kc, vc, bt, cu, cl, 128 ** -0.5)[:n]
+    assert sm100_attn.PROMPT_TC_CALLS[0] == calls + 1
+    diff = (alone.double() - both.double()).abs()
+    assert (diff <= 2 ** -7 * torch.maximum(alone.abs(), both.abs()).double()).all() and (diff > 0).double().mean() < 0.01

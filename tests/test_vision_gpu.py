@@ -1,5 +1,5 @@
 """Vision encoder on the GPU: the bf16 CUDA network (tcgen05 GEMMs, LayerNorm / GELU / rotary kernels, non-causal ragged
-attention on the generic kernel) against the fp32 CPU model on the same weights, and a slot read through the pool."""
+attention on the tensor-core prompt kernel) against the fp32 CPU model on the same weights, and a slot read through the pool."""
 import pytest
 import torch
 
