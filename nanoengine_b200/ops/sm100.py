@@ -1127,10 +1127,15 @@ def _portions_call():
     return _PORTIONS[0]
 
 
-def _delta_portions(q, k, v, g, b, A_log, dt_bias, lower_bound, state, slots, cu, fresh, raw, max_n, per_channel, lens=None):
-    """128 x 128 states, the sequences of less than `max_n` new tokens: four tokens at a time from GROUPS_MIN on, one at a time below.  `lens`: lengths of all that are
-    not empty (and not longer), where the host knows them."""
-    step, groups = (True, True) if lens is None else (min(lens) < GROUPS_MIN, max(lens) >= GROUPS_MIN)
+def _delta_portions(q, k, v, g, b, A_log, dt_bias, lower_bound, state, slots, cu, fresh, raw, max_n, per_channel, cu_host=None):
+    """128 x 128 states, the sequences of less than `max_n` new tokens: four tokens at a time from GROUPS_MIN on, one at a time below.  `cu_host`: their boundaries
+    where the host knows them; a captured call launches both forms, since the boundaries on the device may be others when it is replayed."""
+    step = groups = True
+    if cu_host is not None and not torch.cuda.is_current_stream_capturing():
+        lens = [e - s for s, e in zip(cu_host, cu_host[1:]) if s < e < s + max_n]
+        if not lens:
+            return
+        step, groups = bool(min(lens) < GROUPS_MIN), bool(max(lens) >= GROUPS_MIN)
     _ck(_portions_call()(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), b.data_ptr(), q.stride(0), v.stride(0), b.stride(0), A_log.data_ptr(),
                          dt_bias.data_ptr(), lower_bound, state.data_ptr(), slots.data_ptr(), cu.data_ptr(), fresh.data_ptr(), raw.data_ptr(), q.shape[0],
                          cu.numel() - 1, q.shape[1], v.shape[1], GROUPS_MIN, max_n, step, groups, per_channel, torch.cuda.current_stream().cuda_stream),
@@ -1148,9 +1153,10 @@ def _gdn_step(q, k, v, a, b, A_log, dt_bias, state, slots, cu, fresh, z, norm_w,
 
 def gdn_recurrent(q, k, v, a, b, A_log, dt_bias, state, slots, cu_seqlens, fresh, z, norm_w, eps: float, max_q_len: int = 1,
                   cu_host=None) -> torch.Tensor:
-    """Gated delta rule + gated RMSNorm.  Sequences shorter than `ref.GDN_CHUNK_MIN_TOKENS` new tokens (decode, verification,
-    short chunks) run in the recurrent kernel that keeps the state in registers; longer ones take the chunked form (`delta_chunk.cu` for
-    128 x 128 states, batched matrix products otherwise), and need the host copy of the sequence boundaries (`cu_host`)."""
+    """Gated delta rule + gated RMSNorm.  Sequences shorter than `ref.GDN_CHUNK_MIN_TOKENS` new tokens (decode, verification, short chunks) run in recurrent
+    kernels that keep the state in registers (128 x 128 states from GROUPS_MIN tokens on four at a time, where `max_q_len` or the mean says that there may be
+    some); longer ones take the chunked form (`delta_chunk.cu` for 128 x 128 states, batched matrix products otherwise), and need the host copy of the sequence
+    boundaries (`cu_host`)."""
     T, Hk, Dk = q.shape
     Hv, Dv = v.shape[1], v.shape[2]
     for t in (q, k, v, z):
@@ -1174,9 +1180,7 @@ def gdn_recurrent(q, k, v, a, b, A_log, dt_bias, state, slots, cu_seqlens, fresh
             _ck(lib().ne_delta_chunk(_p(q), _p(k), _p(v), _c.c_longlong(q.stride(0)), _c.c_longlong(v.stride(0)), _p(a), _p(b), _c.c_longlong(a.stride(0)),
                                      _p(A_log), _p(dt_bias), _p(state), _p(slots), _p(cu), _p(fresh), _p(raw), _p(work), _c.c_int(T), _c.c_int(cu.numel() - 1),
                                      _c.c_int(chunks), _c.c_int(Hk), _c.c_int(Hv), _c.c_int(skip), _st()), "ne_delta_chunk")
-            short = [e - s for s, e in zip(cu_host, cu_host[1:]) if s < e < s + skip]
-            if short:
-                _delta_portions(q, k, v, a, b, A_log, dt_bias, 0.0, state, slots, cu, fresh, raw, skip, False, short)
+            _delta_portions(q, k, v, a, b, A_log, dt_bias, 0.0, state, slots, cu, fresh, raw, skip, False, cu_host)
             return rmsnorm_gated(raw, z, norm_w, eps, out).view(T, Hv * Dv)
         rep = Hv // Hk
         g, beta = ref.gdn_gates(a, b, A_log, dt_bias)
@@ -1193,7 +1197,7 @@ def gdn_recurrent(q, k, v, a, b, A_log, dt_bias, state, slots, cu_seqlens, fresh
             rmsnorm_gated(o, z[s:e], norm_w, eps, out[s:e])
     elif (max_q_len >= GROUPS_MIN or T >= GROUPS_MIN * (cu.numel() - 1)) and _delta_rows16(q, k, v, state):
         raw = torch.empty(T, Hv, Dv, dtype=torch.float32, device=q.device)
-        _delta_portions(q, k, v, a, b, A_log, dt_bias, 0.0, state, slots, cu, fresh, raw, skip, False, None if cu_host is None or T == 0 else [e - s for s, e in zip(cu_host, cu_host[1:]) if s < e] or None)
+        _delta_portions(q, k, v, a, b, A_log, dt_bias, 0.0, state, slots, cu, fresh, raw, skip, False, cu_host)
         return rmsnorm_gated(raw, z, norm_w, eps, out).view(T, Hv * Dv)
     raw = bool(lib().ne_gdn_step_raw_only(_c.c_int(Dk), _c.c_int(Dv)))     # large states: several CTAs per head, norm in its own kernel
     if raw and max_q_len >= ref.GDN_CHUNK_MIN_TOKENS:

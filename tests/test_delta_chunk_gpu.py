@@ -202,3 +202,27 @@ def test_a_sequence_does_not_depend_on_its_batch(per_channel, n, others):
         alone = run(own, [n], one, slots[at: at + 1], fresh[at: at + 1], host)
         batch = run(slice(0, t), lens, all_, slots, fresh, host)
         assert torch.equal(batch[own], alone) and torch.equal(all_[slots[at].long()], one[slots[at].long()])
+
+
+@pytest.mark.parametrize("first,then", [([7, 9, 20], [1, 3, 32]), ([2, 3, 4, 6], [1, 12, 1, 1]), ([70, 40], [75, 35]), ([100, 1, 9], [66, 40, 4])])
+def test_a_captured_call_follows_the_boundaries_on_the_device(first, then):
+    from nanoengine_b200.ops import sm100
+    hk, hv = 1, 2
+    gen, r, q, k, v, state, slots, fresh, cu, z, w = _inputs(first, hk, hv, 15)
+    t, longest = sum(first), max(*first, *then)
+    a, b = r(t, 2 * hv).to(torch.bfloat16).split(hv, 1)
+    A, bias = torch.zeros(hv, device="cuda"), torch.zeros(hv, device="cuda")
+    ends = torch.tensor(cu, dtype=torch.int32, device="cuda")
+    st = state.clone()
+    run = lambda st, ends, host: sm100.gdn_recurrent(q, k, v, a, b, A, bias, st, slots, ends, fresh, z, w, 1e-6, longest, host)             # noqa: E731
+    run(state.clone(), ends, cu)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = run(st, ends, cu)
+    other = [0] + torch.tensor(then).cumsum(0).tolist()
+    ends.copy_(torch.tensor(other, dtype=torch.int32))
+    st.copy_(state)
+    graph.replay()
+    want_state = state.clone()
+    want = run(want_state, torch.tensor(other, dtype=torch.int32, device="cuda"), other)
+    assert torch.equal(got, want) and torch.equal(st, want_state)
